@@ -251,17 +251,30 @@ __global__ void __launch_bounds__(C2P_THREADS) k_mlp_bracket(Par p, Z zones, lon
   mlp_tc_finish(&S->tile);
 }
 
-// Per-zone statistics into the block's shared counters.
-__device__ __forceinline__ void c2p_tally(unsigned int *s_hist, unsigned long long *s_cnt, const C2POut &out,
-                                          bool setup_ok, bool success) {
-  const int h = out.iterations < PHX_C2P_HIST ? out.iterations : PHX_C2P_HIST - 1;
-  atomicAdd(&s_hist[h], 1u);
-  atomicAdd(&s_cnt[0], (unsigned long long)out.iterations);
-  atomicAdd(&s_cnt[1], (unsigned long long)out.evals);
-  if (!success) atomicAdd(&s_cnt[2], 1ull);
-  if (setup_ok && !out.bracketed) atomicAdd(&s_cnt[3], 1ull);
-  atomicAdd(&s_cnt[4], 1ull);
-  if (out.learned) atomicAdd(&s_cnt[5], 1ull);
+// A warp's zones into the block's shared counters (every lane of the warp
+// calls it; counted: the lane finished a zone).  Sums over the warp first:
+// lane-by-lane 64-bit shared atomics on one address serialise.
+__device__ __forceinline__ void c2p_tally(unsigned int *s_hist, unsigned long long *s_cnt, bool counted,
+                                          const C2POut &out, bool setup_ok, bool success) {
+  constexpr unsigned all = 0xffffffffu;
+  const int h = counted ? (out.iterations < PHX_C2P_HIST ? out.iterations : PHX_C2P_HIST - 1) : -1;
+  const unsigned same = __match_any_sync(all, h);
+  const int lane = threadIdx.x & 31;
+  if (counted && lane == __ffs(same) - 1) atomicAdd(&s_hist[h], (unsigned)__popc(same));
+  const unsigned it = __reduce_add_sync(all, counted ? (unsigned)out.iterations : 0u);
+  const unsigned ev = __reduce_add_sync(all, counted ? (unsigned)out.evals : 0u);
+  const unsigned failed = __ballot_sync(all, counted && !success);
+  const unsigned unbr = __ballot_sync(all, counted && setup_ok && !out.bracketed);
+  const unsigned zones = __ballot_sync(all, counted);
+  const unsigned lrn = __ballot_sync(all, counted && out.learned);
+  if (lane == 0 && zones) {
+    atomicAdd(&s_cnt[0], (unsigned long long)it);
+    atomicAdd(&s_cnt[1], (unsigned long long)ev);
+    if (failed) atomicAdd(&s_cnt[2], (unsigned long long)__popc(failed));
+    if (unbr) atomicAdd(&s_cnt[3], (unsigned long long)__popc(unbr));
+    atomicAdd(&s_cnt[4], (unsigned long long)__popc(zones));
+    if (lrn) atomicAdd(&s_cnt[5], (unsigned long long)__popc(lrn));
+  }
 }
 
 __device__ __forceinline__ void c2p_flush_stats(DevStats *stats, const unsigned int *s_hist,
@@ -272,20 +285,20 @@ __device__ __forceinline__ void c2p_flush_stats(DevStats *stats, const unsigned 
   if (threadIdx.x == 0) {
     atomicAdd(&stats->iterations, s_cnt[0]);
     atomicAdd(&stats->residual_evals, s_cnt[1]);
-    atomicAdd(&stats->failures, s_cnt[2]);
-    atomicAdd(&stats->unbracketed, s_cnt[3]);
+    if (s_cnt[2]) atomicAdd(&stats->failures, s_cnt[2]);
+    if (s_cnt[3]) atomicAdd(&stats->unbracketed, s_cnt[3]);
     atomicAdd(&stats->zones, s_cnt[4]);
-    atomicAdd(&stats->learned_accepted, s_cnt[5]);
+    if (s_cnt[5]) atomicAdd(&stats->learned_accepted, s_cnt[5]);
   }
 }
 
-// Finish one zone after its root find: unwrap mu, store, fail flag, stats.
+// Finish one zone after its root find: unwrap mu, store, fail flag; returns
+// the zone's success.
 template <class Z, bool MINK>
-__device__ __forceinline__ void c2p_complete(const Par &p, const Z &zones, long long id, const Pt &g, Residual &res,
+__device__ __forceinline__ bool c2p_complete(const Par &p, const Z &zones, long long id, const Pt &g, Residual &res,
                                              double mu, const double rcon[3], const double bu[3],
                                              const double Bprim[3], double bdotr, double U[PHX_NCONS],
-                                             bool setup_ok, const C2POut &out, DevStats *stats, unsigned int *s_hist,
-                                             unsigned long long *s_cnt, unsigned int *err) {
+                                             bool setup_ok, const C2POut &out, unsigned int *err) {
   bool success = false;
   if (setup_ok) {
     double prim[PHX_NPRIM], sig[3];
@@ -299,7 +312,7 @@ __device__ __forceinline__ void c2p_complete(const Par &p, const Z &zones, long 
     if (!out.bracketed) atomicOr(err, ERR_UNBRACKETED);
   }
   zones.store_fail(id, success ? 1.0 : 0.0);
-  if (stats) c2p_tally(s_hist, s_cnt, out, setup_ok, success);
+  return success;
 }
 
 // Zones whose root find is still running after the first kernel's iteration
@@ -328,10 +341,11 @@ __device__ __forceinline__ void rf_unpack(unsigned long long w, RFState &s) {
 }
 
 // con2prim of zones t0 .. t0 + count - 1, one zone per thread.  LEARNED:
-// the start bracket of zone t is brk[c * count + t - t0].  A lane that has
-// not converged after cap iterations saves its state to rb (warp-aggregated
-// append) and leaves the zone to k_c2p_retry, so that one slow zone does not
-// hold 31 finished lanes of its warp.
+// the start bracket of zone t is brk[c * count + t - t0].  Zones that the fast
+// root does not accept (exact build: lanes that have not converged after cap
+// iterations, with their saved state) are appended to rb (warp-aggregated)
+// and left to k_c2p_retry, so that one slow zone does not hold 31 finished
+// lanes of its warp.
 template <class Z, bool MINK, bool LEARNED>
 __global__ void __launch_bounds__(C2P_THREADS) k_c2p(Par p, Z zones, long long t0, long long count,
                                                       const double *brk, int cap, RetryBuf rb, DevStats *stats,
@@ -357,20 +371,24 @@ __global__ void __launch_bounds__(C2P_THREADS) k_c2p(Par p, Z zones, long long t
     setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr);
   }
   const bool run = valid && setup_ok;
-  RFState st;
+  double lb[3] = {0.0, 0.0, 0.0};
   if constexpr (LEARNED) {
-    double lb[3] = {0.0, 0.0, 0.0};
     if (valid && !(guess > 0.0)) {  // brackets exist for cold zones only
       lb[0] = brk[q];
       lb[1] = brk[count + q];
       lb[2] = brk[2 * count + q];
     }
-    rf_start<true>(p, res, run, 0.0, 1.0, guess, lb, st);
-  } else {
-    rf_start<false>(p, res, run, 0.0, 1.0, guess, nullptr, st);
   }
+  C2POut out{0, 0, false, true, false, false};
+#ifdef PHX_EXACT
+  RFState st;
+  rf_start<LEARNED>(p, res, run, 0.0, 1.0, guess, lb, st);
   rf_iterate(p, res, run, st, cap);
   const bool defer = run && rf_running(p, st);
+#else
+  double mu = guess;
+  const bool defer = run && !(c2p_fast_allowed(p) && c2p_fast_root<LEARNED>(p, res, guess, lb, mu, out));
+#endif
   const unsigned m = __ballot_sync(0xffffffffu, defer);
   if (m) {
     const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
@@ -380,19 +398,23 @@ __global__ void __launch_bounds__(C2P_THREADS) k_c2p(Par p, Z zones, long long t
     if (defer) {
       const int pos = base + __popc(m & ((1u << lane) - 1u));
       rb.idx[pos] = (int)q;
+#ifdef PHX_EXACT
       rb.a[pos] = st.a;
       rb.b[pos] = st.b;
       rb.ya[pos] = st.ya;
       rb.yb[pos] = st.yb;
       rb.packed[pos] = rf_pack(st);
+#endif
     }
   }
+  bool success = false;
   if (valid && !defer) {
-    C2POut out{0, 0, false, true, false, false};
+#ifdef PHX_EXACT
     const double mu = rf_result(st, guess, out);
-    c2p_complete<Z, MINK>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, stats, s_hist, s_cnt,
-                          err);
+#endif
+    success = c2p_complete<Z, MINK>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, err);
   }
+  if (stats) c2p_tally(s_hist, s_cnt, valid && !defer, out, setup_ok, success);
   if (stats) c2p_flush_stats(stats, s_hist, s_cnt);
 }
 
@@ -423,19 +445,25 @@ __global__ void __launch_bounds__(C2P_THREADS) k_c2p_retry(Par p, Z zones, long 
       double x1, x2, x3;
       zones.template load<MINK>(t0 + rb.idx[k], id, g, U, x1, x2, x3, guess);
       setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr);
+#ifdef PHX_EXACT
       st.a = rb.a[k];
       st.b = rb.b[k];
       st.ya = rb.ya[k];
       st.yb = rb.yb[k];
       rf_unpack(rb.packed[k], st);
+#endif
     }
+#ifndef PHX_EXACT  // the fast root was not accepted: the reference's iteration from its start
+    rf_start<false>(p, res, valid && setup_ok, 0.0, 1.0, guess, nullptr, st);
+#endif
     rf_iterate(p, res, valid && setup_ok, st, p.c2p_max_iter);
+    C2POut out{0, 0, false, true, false, false};
+    bool success = false;
     if (valid) {
-      C2POut out{0, 0, false, true, false, false};
       const double mu = rf_result(st, guess, out);
-      c2p_complete<Z, MINK>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, stats, s_hist,
-                            s_cnt, err);
+      success = c2p_complete<Z, MINK>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, err);
     }
+    if (stats) c2p_tally(s_hist, s_cnt, valid, out, setup_ok, success);
   }
   if (stats) c2p_flush_stats(stats, s_hist, s_cnt);
 }
@@ -634,26 +662,21 @@ __global__ void __launch_bounds__(C2P_THREADS) kb_c2p(Par p, const BView *views,
       zones.template load<MINK>(q, id, g, U, x1, x2, x3, guess);
       setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr);
     }
-    RFState st;
+    double lb[3] = {0.0, 0.0, 0.0};
     if constexpr (LEARNED) {
       const long long stride = (long long)nitems * C2P_THREADS, o = (long long)it * C2P_THREADS + threadIdx.x;
-      double lb[3] = {0.0, 0.0, 0.0};
       if (valid && !(guess > 0.0)) {  // brackets exist for cold zones only
         lb[0] = brk[o];
         lb[1] = brk[stride + o];
         lb[2] = brk[2 * stride + o];
       }
-      rf_start<true>(p, res, valid && setup_ok, 0.0, 1.0, guess, lb, st);
-    } else {
-      rf_start<false>(p, res, valid && setup_ok, 0.0, 1.0, guess, nullptr, st);
     }
-    rf_iterate(p, res, valid && setup_ok, st, p.c2p_max_iter);
-    if (valid) {
-      C2POut out{0, 0, false, true, false, false};
-      const double mu = rf_result(st, guess, out);
-      c2p_complete<BoxZones, MINK>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, stats, s_hist,
-                                   s_cnt, err);
-    }
+    C2POut out{0, 0, false, true, false, false};
+    const double mu = c2p_root_warp<LEARNED>(p, res, valid && setup_ok, guess, out, lb);
+    bool success = false;
+    if (valid)
+      success = c2p_complete<BoxZones, MINK>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, err);
+    if (stats) c2p_tally(s_hist, s_cnt, valid, out, setup_ok, success);
   }
   if (stats) c2p_flush_stats(stats, s_hist, s_cnt);
 }
@@ -705,14 +728,10 @@ __global__ void __launch_bounds__(C2P_THREADS) kb_ox1_inflow(Par p, const BView 
       zones.template load<false>(q, id, g, U, x1, x2, x3, guess);
       setup_ok = c2p_setup<false>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr);
     }
-    RFState st;
-    rf_start<false>(p, res, valid && setup_ok, 0.0, 1.0, guess, nullptr, st);
-    rf_iterate(p, res, valid && setup_ok, st, p.c2p_max_iter);
-    if (!valid) continue;
     C2POut out{0, 0, false, true, false, false};
-    const double mu = rf_result(st, guess, out);
-    c2p_complete<BoxZones, false>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, nullptr,
-                                  nullptr, nullptr, err);
+    const double mu = c2p_root_warp<false>(p, res, valid && setup_ok, guess, out);
+    if (!valid) continue;
+    c2p_complete<BoxZones, false>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, err);
     double *P = bv.prim + id;
     const long long vs = bv.vs;
     double vel[3] = {P[PHX_PVEL * vs], P[(PHX_PVEL + 1) * vs], P[(PHX_PVEL + 2) * vs]};

@@ -458,6 +458,353 @@ __device__ __forceinline__ double regula_falsi_warp(const Par &p, Residual &res,
   return rf_result(s, guess, out);
 }
 
+#ifndef PHX_EXACT
+// ------------------------------------------------ production root find
+// The residual is FP64-bound: an FP64 instruction holds a sub-partition's
+// FP64 pipe for 64-76 cycles, an FP32 instruction takes one to two.  So the
+// search for the root runs in FP32: a safeguarded Newton iteration with the
+// analytic derivative, then two Newton steps on the residual in pairs of
+// floats (48 bits), which bring mu to about 1e-13.  One FP64 residual
+// evaluation corrects that value; the correction times the slope's own
+// error is what is left, and the zone is accepted when it is below the
+// caller's tolerance (otherwise secant steps with further FP64 evaluations
+// follow).  A zone that does not pass these tests (floors or caps switching
+// at the root, values outside the FP32 range, NaN) takes the reference's
+// bracketed iteration instead.
+// Measured against the bracketed iteration in FP64 (GB300): 1.2e7 cold
+// Kerr-Schild zones at tolerance 1e-13 30.0 -> 7.4 ms (12.8 -> 1.05 FP64
+// residual evaluations per zone), a 136^3 Minkowski block from stale mu
+// 3.90 -> 1.15 ms (7.0 -> 1.0 evaluations), 1000 cold zones 96 -> 40 us; the
+// root's error against the sampled state 3e-14 -> 5e-15.
+
+// a > b for doubles by their bit patterns (no NaN; -0 sorts below +0): an FP64
+// comparison holds the FP64 pipe like an FMA.
+__device__ __forceinline__ bool gt_bits(double a, double b) {
+  long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  x ^= (x >> 63) & 0x7fffffffffffffffll;
+  y ^= (y >> 63) & 0x7fffffffffffffffll;
+  return x > y;
+}
+
+// float from a double by bit operations (a conversion instruction holds the
+// FP64 pipe): truncated, 0 below and +-max above the FP32 normal range.
+__device__ __forceinline__ float d2f_bits(double x) {
+  const int hi = __double2hiint(x);
+  const int mag = hi & 0x7fffffff;
+  unsigned m = ((unsigned)(mag - 0x38000000) << 3) | ((unsigned)__double2loint(x) >> 29);
+  if (mag < 0x38100000) m = 0u;
+  if (mag >= 0x47e00000) m = 0x7f7fffffu;
+  return __int_as_float((int)(m | (hi & 0x80000000)));
+}
+// double from a normal float (exact), by bit operations
+__device__ __forceinline__ double f2d_bits(float f) {
+  const int b = __float_as_int(f);
+  const int mag = b & 0x7fffffff;
+  const int hi = mag < 0x00800000 ? 0 : (mag >> 3) + 0x38000000;
+  return __hiloint2double(hi | (b & 0x80000000), mag < 0x00800000 ? 0 : (b << 29));
+}
+
+__device__ __forceinline__ float rcp_f32(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_f32(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Pairs of floats h + l (|l| <= ulp(h) / 2): the error-free sum of Knuth and
+// Dekker's product with an FMA, the usual double-word algorithms on them.
+struct FF {
+  float h, l;
+};
+__device__ __forceinline__ FF ff_quick(float a, float b) {  // |a| >= |b|
+  const float s = __fadd_rn(a, b);
+  return {s, __fsub_rn(b, __fsub_rn(s, a))};
+}
+__device__ __forceinline__ FF ff_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), v = __fsub_rn(s, a);
+  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, v)), __fsub_rn(b, v))};
+}
+__device__ __forceinline__ FF ff_add(FF a, FF b) {
+  FF s = ff_sum(a.h, b.h);
+  return ff_quick(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
+}
+__device__ __forceinline__ FF ff_addf(FF a, float b) {
+  FF s = ff_sum(b, a.h);
+  return ff_quick(s.h, __fadd_rn(s.l, a.l));
+}
+__device__ __forceinline__ FF ff_neg(FF a) { return {-a.h, -a.l}; }
+__device__ __forceinline__ FF ff_mul(FF a, FF b) {
+  const float p = __fmul_rn(a.h, b.h);
+  float e = __fmaf_rn(a.h, b.h, -p);
+  e = __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, e));
+  return ff_quick(p, e);
+}
+__device__ __forceinline__ FF ff_rcp(FF a) {
+  const float r = rcp_f32(a.h);
+  float e = __fmaf_rn(-a.h, r, 1.0f);
+  e = __fmaf_rn(-a.l, r, e);
+  return ff_quick(r, __fmul_rn(r, __fmaf_rn(e, e, e)));
+}
+__device__ __forceinline__ FF ff_rsqrt(FF a) {
+  const float y = rsqrt_f32(a.h);
+  const float p = __fmul_rn(y, y), pe = __fmaf_rn(y, y, -p);
+  float g = __fmaf_rn(-a.h, p, 1.0f);
+  g = __fmaf_rn(-a.h, pe, __fmaf_rn(-a.l, p, g));
+  return ff_quick(y, __fmul_rn(y, __fmul_rn(g, __fmaf_rn(0.375f, g, 0.5f))));
+}
+// the leading 47 bits of a double: h truncated, l the next 23 bits (0 where it
+// would be subnormal)
+__device__ __forceinline__ FF ff_bits(double x) {
+  FF r;
+  r.h = d2f_bits(x);
+  const int b = __float_as_int(r.h), ex = b & 0x7f800000;
+  const int sg = b & 0x80000000;
+  const int el = ex - (23 << 23);
+  const unsigned rem = ((unsigned)__double2loint(x) >> 6) & 0x7fffffu;
+  const float unit = __int_as_float(el | sg);
+  r.l = (el > 0 && (b & 0x7fffffff) != 0x7f7fffff) ? __fsub_rn(__int_as_float(el | sg | (int)rem), unit) : 0.0f;
+  return r;
+}
+
+// The residual with Phat = gm1 rho e written out: the reference's ahat is
+// gm1 e / (1 + e) and (1 + ahat)(1 + e) = 1 + Gamma e, so the density enters
+// only through the floors; x rbarsq as x (mu rbsq + x (rsq + mu rbsq)).
+//   eval:  FP32 and the derivative
+//   evalp: pairs of floats
+//   eval64: FP64; 38 arithmetic instructions and integer comparisons
+struct FastResidual {
+  FF q, hb, rsq, rbsq, v0sq, gm1, bsq;  // q: q - bsq / 2, hb: -bsq_rpsq / 2
+  float efl, emax;
+  double qh, efl64;
+  __device__ __forceinline__ FastResidual(const Par &p, const Residual &r) {
+    qh = fma(-0.5, r.bsq, r.q);
+    q = ff_bits(qh);
+    bsq = ff_bits(r.bsq);
+    hb = ff_bits(r.bsq_rpsq);
+    hb.h *= -0.5f;
+    hb.l *= -0.5f;
+    rsq = ff_bits(r.rsq);
+    rbsq = ff_bits(r.rbsq);
+    v0sq = ff_bits(r.v0sq);
+    gm1 = ff_bits(p.gm1);
+    double rho = r.rho_floor;  // ExpX1RhoU: the sie floor at the density floor, its largest value
+    floors_from(p, r.fl, rho, efl64);
+    efl64 *= p.fsf;
+    efl = d2f_bits(efl64);
+    emax = d2f_bits(r.e_max);
+  }
+  __device__ __forceinline__ float eval(float mu, float &df) const {
+    const float x = rcp_f32(fmaf(mu, bsq.h, 1.0f));
+    const float dx = -bsq.h * x * x;
+    const float mr = mu * rbsq.h, u = rsq.h + mr;
+    const float w = fmaf(x, u, mr);
+    const float rb = x * w;
+    const float drb = fmaf(dx, fmaf(x, u, w), x * fmaf(x, rbsq.h, rbsq.h));
+    const float mux = mu * x;
+    const float qb = fmaf(mux * mux, hb.h, q.h);
+    const float dqb = 2.0f * mux * fmaf(mu, dx, x) * hb.h;
+    const float mrb = mu * rb, dmrb = fmaf(mu, drb, rb);
+    float v2 = mu * mrb, dv2 = fmaf(mu, dmrb, mrb);
+    if (v2 > v0sq.h) {
+      v2 = v0sq.h;
+      dv2 = 0.0f;
+    }
+    const float om = 1.0f - v2;
+    const float W = rsqrt_f32(om), iW = om * W;
+    const float A = qb - mrb, dA = dqb - dmrb;
+    const float dW = 0.5f * W * W * W * dv2, diW = -0.5f * W * dv2;
+    float e = fmaf(W, A, W - 1.0f), de = fmaf(dW, A + 1.0f, W * dA);
+    if (e <= efl) {
+      e = efl;
+      de = 0.0f;
+    } else if (e > emax) {
+      e = emax;
+      de = 0.0f;
+    }
+    const float P = fmaxf(gm1.h * e, 0.0f);
+    const float dP = gm1.h * e > 0.0f ? gm1.h * de : 0.0f;
+    const float ie = rcp_f32(1.0f + e);
+    const float a = P * ie, da = (dP - a * de) * ie;
+    const float h = 1.0f + e + P, dh = de + dP;
+    const float nua = h * iW, nub = (1.0f + a) * (1.0f + A);
+    const float dnu = nua > nub ? fmaf(dh, iW, h * diW) : fmaf(da, 1.0f + A, (1.0f + a) * dA);
+    const float g = rcp_f32(fmaxf(nua, nub) + mrb);
+    df = fmaf(g * g, dnu + dmrb, 1.0f);
+    return mu - g;
+  }
+  __device__ __forceinline__ float evalp(FF mu) const {
+    const FF x = ff_rcp(ff_addf(ff_mul(mu, bsq), 1.0f));
+    const FF mr = ff_mul(mu, rbsq);
+    const FF rb = ff_mul(x, ff_add(mr, ff_mul(x, ff_add(rsq, mr))));
+    const FF mux = ff_mul(mu, x);
+    const FF mrb = ff_mul(mu, rb);
+    const FF A = ff_add(ff_add(q, ff_mul(ff_mul(mux, mux), hb)), ff_neg(mrb));
+    FF v2 = ff_mul(mu, mrb);
+    if (v2.h > v0sq.h || (v2.h == v0sq.h && v2.l > v0sq.l)) v2 = v0sq;
+    const FF om = ff_addf(ff_neg(v2), 1.0f);
+    const FF W = ff_rsqrt(om), iW = ff_mul(om, W);
+    FF e = ff_add(ff_mul(W, A), ff_addf(W, -1.0f));
+    if (e.h <= efl) {
+      e = {efl, 0.0f};
+    } else if (e.h > emax) {
+      e = {emax, 0.0f};
+    }
+    const FF e1 = ff_addf(e, 1.0f);
+    const FF h = e.h > 0.0f ? ff_add(e1, ff_mul(gm1, e)) : e1;
+    const FF nua = ff_mul(h, iW), nub = ff_mul(ff_mul(h, ff_rcp(e1)), ff_addf(A, 1.0f));
+    const FF g = ff_rcp(ff_add(nua.h > nub.h ? nua : nub, mrb));
+    return __fadd_rn(__fsub_rn(mu.h, g.h), __fsub_rn(mu.l, g.l));
+  }
+  // false (the reference's expressions apply): a density small enough for the
+  // reference's bound on h rho, an energy below 0, ExpX1RhoU's floor active
+  __device__ __forceinline__ bool eval64(const Par &p, const Residual &r, double mu, double &f) const {
+    const double x = rcp_p(fma(mu, r.bsq, 1.0));
+    const double mr = mu * r.rbsq;
+    const double rb = x * fma(x, r.rsq + mr, mr);
+    const double mux = mu * x;
+    const double mrb = mu * rb;
+    const double A = fma(-0.5 * r.bsq_rpsq, mux * mux, qh) - mrb;
+    double v2 = mu * mrb;
+    if (gt_bits(v2, r.v0sq)) v2 = r.v0sq;
+    const double om = 1.0 - v2;
+    const double W = rsqrt_p(om), iW = om * W;
+    double e = fma(W, A, W - 1.0);
+    if (dexp(e) == 0x7ff) return false;  // NaN or infinity
+    if (!gt_bits(e, efl64)) {
+      if (p.floor_type == PHX_FLOOR_EXPX1_RHO_U) return false;
+      e = efl64;
+    } else if (gt_bits(e, r.e_max)) {
+      e = r.e_max;
+    }
+    if (__double2hiint(e) < 0 || dexp(r.D) + (dexp(iW) - 1023) < 1023 - 46) return false;
+    const double e1 = 1.0 + e;
+    const double h = fma(p.gm1, e, e1);
+    const double nua = h * iW, nub = (h * rcp_p(e1)) * (1.0 + A);
+    f = mu - rcp_p((gt_bits(nua, nub) ? nua : nub) + mrb);
+    return true;
+  }
+};
+
+// Largest number of FP64 evaluations before a zone takes the reference's
+// iteration; iteration caps below it keep the reference's own counting.
+constexpr int C2P_FAST_EVALS = 5;
+__device__ __forceinline__ bool c2p_fast_allowed(const Par &p) {
+  return p.c2p_max_iter >= C2P_FAST_EVALS && p.c2p_tol >= 1e-15 && p.c2p_tol <= 1e-3;
+}
+
+// mu of one zone from its guess (> 0: a previous solution) or, LEARNED, the
+// predicted root lb[0] of a cold zone.  False: not accepted.  mu lies within
+// c2p_tol of the root where true, as the reference's final bracket has it.
+template <bool LEARNED>
+__device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res, double guess, const double *lb,
+                                              double &mu, C2POut &out) {
+  const FastResidual rf(p, res);
+  float lo = 0.0f, hi = 1.0f, s = 1.0f;
+  float m = guess > 0.0 && guess < 1.0 ? d2f_bits(guess) : rsqrt_f32(1.0f + rf.rsq.h);
+  out.learned = false;
+  if constexpr (LEARNED) {
+    if (!(guess > 0.0) && lb[1] >= 0.0 && lb[1] <= lb[0] && lb[0] <= lb[2] && lb[2] <= 1.0) {
+      float d;
+      const float l = d2f_bits(lb[1]), h = d2f_bits(lb[2]);
+      if (rf.eval(l, d) <= 0.0f && rf.eval(h, d) >= 0.0f) {
+        m = d2f_bits(lb[0]);
+        lo = l;
+        hi = h;
+        out.learned = true;
+      }
+    }
+  }
+  float last = 1.0f;
+  for (int it = 0; it < 24; it++) {
+    const float f = rf.eval(m, s);
+    if (f > 0.0f)
+      hi = m;
+    else
+      lo = m;
+    float n = m - f * rcp_f32(s);
+    if (!(n > lo && n < hi)) n = 0.5f * (lo + hi);
+    const float d = fabsf(n - m);
+    m = n;
+    // FP32 rounding reached: the step is at rounding level, or small and no longer shrinking
+    if (d <= 1e-6f * m || (d <= 1e-3f * m && d > 0.5f * last)) break;
+    last = d;
+  }
+  if (!(s > 1e-3f && m > 1e-12f && m <= 1.0f)) return false;
+  FF mp = {m, 0.0f};
+  float is = rcp_f32(s);
+  float fp = rf.evalp(mp);
+#pragma unroll 1
+  for (int it = 0; it < 2; it++) {
+    const float step = fp * is;
+    if (!(fabsf(step) <= 0.5f * m)) return false;
+    const FF mn = ff_addf(mp, -step);
+    const float fn = it == 0 ? rf.evalp(mn) : 0.0f;
+    if (it == 0 && fabsf(step) > 1e-5f * m) is = step * rcp_f32(fp - fn);
+    mp = mn;
+    fp = fn;
+  }
+  double x = f2d_bits(mp.h) + f2d_bits(mp.l), fx;
+  const float tol = d2f_bits(p.c2p_tol);
+  if (!(is > 0.0f && x > 0.0 && x <= 1.0) || !rf.eval64(p, res, x, fx)) return false;
+  float f = d2f_bits(fx);
+  out.iterations = 0;
+  out.evals = 1;
+  // the slope is good to a few parts in 1e3 where a secant confirmed it
+  float gain = 1.0f;
+  for (;;) {
+    const float step = f * is;
+    const float as = fabsf(step);
+    const double xn = x - f2d_bits(step);
+    out.iterations++;
+    if (!(as <= 0.5f * m)) return false;
+    if (as <= gain * tol) {  // the error after this step: the step times the slope's relative error
+      mu = xn < 1.0 ? xn : 1.0;
+      return xn > 0.0;
+    }
+    if (out.evals >= C2P_FAST_EVALS || !(xn > 0.0 && xn <= 1.0) || !rf.eval64(p, res, xn, fx)) return false;
+    const float fn = d2f_bits(fx);
+    out.evals++;
+    if (as > 1e-9f * m) {
+      const float isec = step * rcp_f32(f - fn);
+      if (!(isec > 0.0f && isec < 1e3f)) return false;
+      gain = fabsf(is * rcp_f32(isec) - 1.0f) <= 0.03125f ? 16.0f : 1.0f;
+      is = isec;
+    }
+    x = xn;
+    f = fn;
+  }
+}
+#endif
+
+// The root of one zone per lane, warp-synchronous: the production build's
+// fast root where it is accepted, the reference's iteration elsewhere.
+template <bool LEARNED>
+__device__ __forceinline__ double c2p_root_warp(const Par &p, Residual &res, bool valid, double guess, C2POut &out,
+                                                const double *lb = nullptr) {
+#ifndef PHX_EXACT
+  bool need = valid;
+  double mu = guess;
+  if (valid && c2p_fast_allowed(p)) need = !c2p_fast_root<LEARNED>(p, res, guess, lb, mu, out);
+  if (!__any_sync(0xffffffffu, need)) return mu;
+  C2POut slow{0, 0, false, true, false, false};
+  const double ms = regula_falsi_warp<false>(p, res, need, 0.0, 1.0, guess, slow);
+  if (need) {
+    out.iterations = slow.iterations;
+    out.evals = slow.evals;
+    out.bracketed = slow.bracketed;
+    out.learned = false;
+    mu = ms;
+  }
+  return mu;
+#else
+  return regula_falsi_warp<LEARNED>(p, res, valid, 0.0, 1.0, guess, out, lb);
+#endif
+}
+
 // Unwrap mu into primitives (con2prim_robust.hpp:381-452).
 // prim[] receives PHX_NPRIM values (B slots only when mhd), U[] may be
 // rewritten by p2c when bounds were used; sig[3] receives signal speeds.
