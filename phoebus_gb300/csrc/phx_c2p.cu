@@ -468,13 +468,6 @@ __global__ void __launch_bounds__(C2P_THREADS) k_c2p_retry(Par p, Z zones, long 
   if (stats) c2p_flush_stats(stats, s_hist, s_cnt);
 }
 
-static int num_sms() {
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  return nsm > 0 ? nsm : 1;
-}
-
 template <class Z, bool MINK>
 static void launch_bracket_any(const Par &p, const Z &z, long long t0, long long count, const MlpPacked *mlp,
                                double *brk, unsigned int *err, cudaStream_t s) {
@@ -485,7 +478,7 @@ static void launch_bracket_any(const Par &p, const Z &z, long long t0, long long
     attr = true;
   }
   long long grid = (count + C2P_THREADS - 1) / C2P_THREADS;
-  const long long cap = (long long)num_sms() * 8;
+  const long long cap = (long long)sm_count() * 8;
   if (grid > cap) grid = cap;
   k_mlp_bracket<Z, MINK><<<(unsigned)grid, C2P_THREADS, sizeof(BracketSmem), s>>>(p, z, t0, count, mlp, brk, err);
 }
@@ -509,7 +502,7 @@ static void launch_c2p_any(const Par &p, const Z &z, long long n, const MlpPacke
   static const int cap_learned = cap_from_env("PHX_C2P_CAP_LEARNED", 6);
   const int cap = mlp ? cap_learned : cap_plain;
   RetryBuf rb{scr.count, scr.idx, scr.a, scr.b, scr.ya, scr.yb, scr.packed};
-  const unsigned retry_grid = (unsigned)num_sms() * 4;
+  const unsigned retry_grid = (unsigned)sm_count() * 4;
   for (long long t0 = 0; t0 < n; t0 += C2P_CHUNK) {
     const long long m = n - t0 < C2P_CHUNK ? n - t0 : C2P_CHUNK;
     const long long grid = (m + C2P_THREADS - 1) / C2P_THREADS;

@@ -15,6 +15,7 @@
 
 #include "../../include/phx_fluid.h"
 #include "phx_math.h"
+#include "phx_weno.cuh"
 
 namespace phx {
 
@@ -588,104 +589,60 @@ __device__ __forceinline__ void recon_weno5z(double q0, double q1, double q2, do
   qr = alpha_lin * qr + (1.0 - alpha_lin) * (q2 - 0.5 * dq);
 }
 // ---- production-build WENO5-Z: same mathematics, fewer FP64 instructions.
-// WENO5-Z as reconstruction.hpp:127-183, rearranged.
-//  - The nonlinear weights are gamma_k bp_k, bp_k = 1 + tau5 / beta_k,
-//    normalised by their sums S_l, S_r; the three 1/beta_k come from one
-//    reciprocal of beta0 beta1 beta2.  (The reference's + eps on a weight is
-//    below half an ulp of gamma_k bp_k >= 0.1 and drops out.)
-//  - The blend factor: with normalised weights w_k = gamma_k bp_k / S,
-//    alpha = 3 w0 w1 w2 / (g2 w0 w1 + g1 w0 w2 + g0 w1 w2) = 3 / (S R) with
-//    R = sum_k 1/bp_k, the same for both faces, so the harmonic mean
-//    alpha_lin = 2 alpha_l alpha_r / (alpha_l + alpha_r) = 6 / (R (S_l + S_r)).
-//    1/bp_k = beta_k / (beta_k + tau5): with M the larger of beta0, beta2 and
-//    m the smaller, beta_m + tau5 = beta_M, so 1/bp_m = beta_m / beta_M from
-//    the reciprocal above, and 1/bp_M, 1/bp_1 share one reciprocal of
-//    (2 beta_M - beta_m)(beta1 + tau5).  (The reference's + eps on alpha_l,
-//    alpha_r moves alpha_lin only where alpha_lin < 1e-90.)  alpha_lin and
-//    the weights' normalisations 1 / S_l, 1 / S_r come from one reciprocal of
-//    R (S_l + S_r) S_l S_r.
+// WENO5-Z as reconstruction.hpp:127-183, rearranged; the weights and the blend
+// factor alpha_lin come from phx_weno.cuh.  With normalised weights
+// w_k = gamma_k bp_k / S (bp_k = 1 + tau5 / beta_k; the reference's + eps on
+// a weight is below half an ulp of gamma_k bp_k >= 0.1 and drops out),
+// alpha = 3 w0 w1 w2 / (g2 w0 w1 + g1 w0 w2 + g0 w1 w2) = 3 / (S R) with
+// R = sum_k 1/bp_k, the same for both faces, so the harmonic mean is
+// alpha_lin = 6 / (R (S_l + S_r)).
+//  - The candidates are q2 + (a_k +- 3 b_k) / 12; the blend
+//    alpha q + (1 - alpha) p with p = q2 +- dq2 / 4 is
+//    p -+ (alpha / 4) dq2 + sum_k W_k (a_k +- 3 b_k).
 //  - The MC slope of the blend, mc(q2 - q1, q3 - q2, 2), doubled, on the
 //    integer pipe: the sign test, the minima of magnitudes and the power-of-two
 //    scale act on the bit patterns; the sum dm + dp is the slope b1 = q3 - q1
 //    the smoothness indicator already forms.
-// Three reciprocals (three FP64 instructions each) and about 90 FP64
-// instructions for both face states.  Every intermediate stays in the normal
-// range for |q| < 1e50; outside it (checked on the exponents) the reference
+// 30 FP64 instructions for both face states (81 and three reciprocals with
+// the weights in FP64): 256^3 fluxes in all three directions 99.0 -> 69.6 ms,
+// and 56.6 ms with the flux kernels' loop over the variables rolled.
+// Where the weights are refused (values beyond 1e270, not finite) the reference
 // sequence is used.
 __device__ __forceinline__ void recon_weno5z_fast(double q0, double q1, double q2, double q3, double q4,
                                                   double &ql, double &qr) {
-  constexpr double g0 = 0.1, g1 = 0.6, g2 = 0.3;
-  constexpr double eps = 1e-100;
-  constexpr double t13 = 13.0 / 3.0;
-  // second differences a_k and one-sided slopes b_k of the three stencils;
-  // beta_k = 13/3 a_k^2 + b_k^2 + eps with eps folded into the b^2 product.
-  // These keep the reference's operation order: in near-flat regions the
-  // weights follow the rounding of a_k and b_k (differences of nearly equal
-  // indicators), and forming them from first differences instead moved
-  // signal speeds of a 256^3 shear layer 1.7e-12 away from the reference's.
+  // second differences a_k and one-sided slopes b_k of the three stencils, in
+  // the reference's operation order: in near-flat regions the weights follow
+  // the rounding of a_k and b_k (differences of nearly equal indicators), and
+  // forming them from first differences instead moved signal speeds of a
+  // 256^3 shear layer 1.7e-12 away from the reference's.
   const double a0 = q0 - 2 * q1 + q2, b0 = q0 - 4.0 * q1 + 3.0 * q2;
   const double a1 = q1 - 2.0 * q2 + q3, b1 = q3 - q1;
   const double a2 = q2 - 2.0 * q3 + q4, b2 = q4 - 4.0 * q3 + 3.0 * q2;
-  const double beta0 = fma(t13 * a0, a0, fma(b0, b0, eps));
-  const double beta1 = fma(t13 * a1, a1, fma(b1, b1, eps));
-  const double beta2 = fma(t13 * a2, a2, fma(b2, b2, eps));
-  const double d20 = beta2 - beta0;
-  const double tau5 = fabs(d20);
-  const double b01 = beta0 * beta1;
-  const double prod = b01 * beta2;
-  const int ep = dexp(prod);
-  if (ep < 16 || ep > 2030) {  // outside [~1e-303, ~1e303]: reference sequence
+  weno::Weights w;
+  if (!weno::weights(a0, b0, a1, b1, a2, b2, w)) {
     recon_weno5z(q0, q1, q2, q3, q4, ql, qr);
     return;
   }
-  const double rp = rcp_nr(prod);
-  const double t = beta2 * rp;
-  const double ib0 = beta1 * t, ib2 = b01 * rp;  // 1/beta0, 1/beta2
-  const double bp0 = fma(tau5, ib0, 1.0);
-  const double bp1 = fma(tau5, beta0 * t, 1.0);
-  const double bp2 = fma(tau5, ib2, 1.0);
-  const bool big2 = __double2hiint(d20) >= 0;  // beta2 >= beta0
-  const double bM = big2 ? beta2 : beta0, bm = big2 ? beta0 : beta2;
-  const double X1 = fma(2.0, bM, -bm), Y1 = beta1 + tau5;
-  const double X = X1 * Y1;
-  const double wl0 = g0 * bp0, wl1 = g1 * bp1, wl2 = g2 * bp2;
-  const double wr0 = g0 * bp2, wr2 = g2 * bp0;
-  const double Sl = wl0 + wl1 + wl2, Sr = wr0 + wl1 + wr2;
-  const double SS = Sl * Sr, S2 = Sl + Sr;
-  const int ex = dexp(X), eSS = dexp(SS), eS2 = dexp(S2);
-  // R in [1/2, 3] and S_l, S_r >= 1: R S2 SS lies in [1, 2^1021) below the sum bound
-  if (ex < 16 || ex > 2030 || eSS > 2030 || eS2 > 2027 || eSS + eS2 > 3060) {
-    recon_weno5z(q0, q1, q2, q3, q4, ql, qr);
-    return;
-  }
-  const double rx = rcp_nr(X);
-  const double R = fma(bm, big2 ? ib2 : ib0, fma(bM, Y1 * rx, beta1 * (X1 * rx)));
-  // one reciprocal Z = 1 / (R S2 S_l S_r) gives alpha_lin / 4 = 1.5 S_l S_r Z and
-  // the candidates' normalisation with the blend factor folded in:
-  // alpha_lin / (12 S_l) = S_r Z / 2, alpha_lin / (12 S_r) = S_l Z / 2
-  const double Z = rcp_nr(R * S2 * SS);
-  const double aq = (1.5 * SS) * Z;  // alpha_lin / 4
-  const double hZ = 0.5 * Z;
-  const double zl = hZ * Sr, zr = hZ * Sl;
   // 2 mc(q2 - q1, q3 - q2, 2) = copysign(min(|dm + dp|, 4 min(|dm|, |dp|)),
-  // dm + dp) where dm dp > 0, else 0 (finite dm, dp: |q| < 1e50 here)
+  // dm + dp) where dm dp > 0, else 0
   const long long MAG = 0x7fffffffffffffffLL;
   const long long idm = __double_as_longlong(q2 - q1), idp = __double_as_longlong(q3 - q2);
   const long long isum = __double_as_longlong(b1);
   const long long adm = idm & MAG, adp = idp & MAG, asum = isum & MAG;
   const bool same = ((idm ^ idp) >= 0) && adm != 0 && adp != 0;
   const long long a4 = (adm < adp ? adm : adp) + (2LL << 52);
-  const double dq2 = same ? __longlong_as_double((asum < a4 ? asum : a4) | (isum & ~MAG)) : 0.0;
-  // candidate values as q2 plus a twelfth of a_k +- 3 b_k: for ql (upper
-  // face) (a0 + 3 b0), (a1 + 3 b1), (a2 - 3 b2); for qr (lower face, the
-  // mirrored stencils) (a2 + 3 b2), (a1 - 3 b1), (a0 - 3 b0); the weights sum
-  // to one, so sum_k w_k c_k = q2 + sum_k w_k (c_k - q2).  Then the blend
-  // alpha q + (1 - alpha) p with p = q2 +- dq2 / 4 as p -+ (alpha / 4) dq2 +
-  // alpha (q - q2), alpha (q - q2) = (sum_k w_k (a_k +- 3 b_k)) alpha / (12 S).
-  const double sl = wl0 * fma(3.0, b0, a0) + wl1 * fma(3.0, b1, a1) + wl2 * fma(-3.0, b2, a2);
-  const double sr = wr0 * fma(3.0, b2, a2) + wl1 * fma(-3.0, b1, a1) + wr2 * fma(-3.0, b0, a0);
-  ql = fma(sl, zl, fma(-aq, dq2, fma(0.25, dq2, q2)));
-  qr = fma(sr, zr, fma(aq, dq2, fma(-0.25, dq2, q2)));
+  // mirrored: the roles of the faces and of the outer stencils change, the
+  // slopes b1 and dq2 change sign
+  const long long flip = w.mirror ? ~MAG : 0;
+  const double ds = same ? __longlong_as_double(((asum < a4 ? asum : a4) | (isum & ~MAG)) ^ flip) : 0.0;
+  const double bs = __longlong_as_double(isum ^ flip);
+  const double am = w.mirror ? a2 : a0, bm = w.mirror ? b2 : b0, aM = w.mirror ? a0 : a2, bM = w.mirror ? b0 : b2;
+  const double t = w.aq * ds;
+  const double sa = fma(w.am, fma(3.0, bm, am), fma(w.a1, fma(3.0, bs, a1), fma(w.aM, fma(-3.0, bM, aM), -t)));
+  const double sb = fma(w.bm, fma(-3.0, bm, am), fma(w.b1, fma(-3.0, bs, a1), fma(w.bM, fma(3.0, bM, aM), t)));
+  const double qa = fma(0.25, ds, q2) + sa, qb = fma(-0.25, ds, q2) + sb;
+  ql = w.mirror ? qb : qa;
+  qr = w.mirror ? qa : qb;
 }
 
 __device__ __forceinline__ double minmod(double a, double b) {

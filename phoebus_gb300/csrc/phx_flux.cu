@@ -91,15 +91,39 @@ __device__ __forceinline__ void face_flux(const Par &p, const BView &b, int k, i
   b.face_sig[(long long)DIR * b.vs + id] = sig;
 }
 
-// ------------------------------------------------------------------ X1
-// Resident CTAs per SM the register allocation of the sweep kernels is
-// bounded for (launch bounds); 1 leaves the compiler free (no spills).
-#ifndef PHX_SWEEP_MINB
-#define PHX_SWEEP_MINB 1
+// Reconstructed states between the loop over the variables and the Riemann
+// solve: one double per thread, variable and slot in shared memory (thread
+// private, no barrier).  With the loop rolled the reconstruction's code is
+// there once -- unrolled over nine variables it no longer fits the
+// instruction cache beside the Riemann solver -- and a thread holds one
+// variable's stencil in registers instead of all of them, which leaves room
+// for the resident warps that hide the integer instructions' latency.
+constexpr int FLUX_THREADS = 128;
+// PLM and constant reconstruction are short enough to unroll (their loads
+// then overlap).  256^3 WENO5-Z, three directions: unrolled with the stencils in
+// registers (228 registers, 12% of the warps resident) 69.6 ms, rolled 56.6 ms.
+template <int RECON>
+constexpr int flux_unroll() {
+  return RECON == PHX_RECON_WENO5Z || RECON == PHX_RECON_MP5 ? 1 : kReconLoad;
+}
+struct FaceStates {
+  double q[kReconLoad][FLUX_THREADS];
+  __device__ __forceinline__ void load(double out[PHX_NRECON]) const {
+#pragma unroll
+    for (int v = 0; v < kReconLoad; v++) out[v] = q[v][threadIdx.x];
+  }
+};
+
+// Resident CTAs per SM the register allocation is bounded for.
+#ifdef PHX_EXACT
+constexpr int flux_minb(bool) { return 1; }
+#else
+constexpr int flux_minb(bool mink) { return mink ? 4 : 3; }
 #endif
 
-constexpr int X1_WARPS = 4;    // warps per CTA
-constexpr int X1_PENCILS = 4;  // (k, j) pencils staged per CTA
+// ------------------------------------------------------------------ X1
+constexpr int X1_WARPS = FLUX_THREADS / 32;  // warps per CTA
+constexpr int X1_PENCILS = 4;                // at most this many (k, j) pencils staged per CTA
 
 // A CTA stages np pencils (kReconLoad primitive rows each) in shared memory
 // with TMA copies completing on one mbarrier.  Its warps then walk the pencils'
@@ -194,7 +218,7 @@ __device__ __forceinline__ bool x1_stage(const BView &b, const X1Range &xr, int 
 
 template <int RECON, bool MINK>
 __device__ __forceinline__ void x1_compute(const Par &p, const BView &b, const X1Range &xr, int p0, int np,
-                                           const double *rows) {
+                                           const double *rows, FaceStates *fs) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarps = (int)(blockDim.x >> 5);
   const int n1t = b.n1t;
@@ -206,61 +230,60 @@ __device__ __forceinline__ void x1_compute(const Par &p, const BView &b, const X
     const int slot = ch * 31 + lane;
     const bool have = slot < nslot;
     const int pp = have ? slot / ncell : 0;
-    const int c = c0 + (have ? slot % ncell : 0);
-    const double *prow = rows + pp * x1_pencil_stride(b);
-    double ql[PHX_NRECON], qr[PHX_NRECON];
-#pragma unroll
-    for (int v = 0; v < kReconLoad; v++) {
-      const double *r = prow + v * n1t;
-      if (have) {
-        if constexpr (RECON == PHX_RECON_WENO5Z || RECON == PHX_RECON_MP5)
-          recon<RECON>(r[c - 2], r[c - 1], r[c], r[c + 1], r[c + 2], ql[v], qr[v]);
-        else if constexpr (RECON == PHX_RECON_LINEAR)
-          recon<RECON>(0.0, r[c - 1], r[c], r[c + 1], 0.0, ql[v], qr[v]);
-        else
-          recon<RECON>(0.0, 0.0, r[c], 0.0, 0.0, ql[v], qr[v]);
-      } else {
-        ql[v] = qr[v] = 0.0;
-      }
+    const int c = c0 + (have ? slot % ncell : 0);  // lanes past the end repeat the first cell
+    const double *r = rows + pp * x1_pencil_stride(b) + c;
+#pragma unroll(flux_unroll<RECON>())
+    for (int v = 0; v < kReconLoad; v++, r += n1t) {
+      double ql, qr;
+      if constexpr (RECON == PHX_RECON_WENO5Z || RECON == PHX_RECON_MP5)
+        recon<RECON>(r[-2], r[-1], r[0], r[1], r[2], ql, qr);
+      else if constexpr (RECON == PHX_RECON_LINEAR)
+        recon<RECON>(0.0, r[-1], r[0], r[1], 0.0, ql, qr);
+      else
+        recon<RECON>(0.0, 0.0, r[0], 0.0, 0.0, ql, qr);
+      fs[0].q[v][threadIdx.x] = __shfl_up_sync(FULL, ql, 1);  // from cell c-1 (same pencil when c > is-1)
+      fs[1].q[v][threadIdx.x] = qr;
     }
-    double left[PHX_NRECON];
-#pragma unroll
-    for (int v = 0; v < kReconLoad; v++) left[v] = __shfl_up_sync(FULL, ql[v], 1);
-    recon_gamma1(p, left, qr);
-    // face of cell c: left state from cell c-1 (same pencil when c > is-1)
-    if (have && lane > 0 && c > c0) {
+    if (have && lane > 0 && c > c0) {  // the face of cell c
       const int pen = p0 + pp;
-      face_flux<MINK, 0>(p, b, xr.klo + pen / xr.nj, xr.jlo + pen % xr.nj, c, left, qr);
+      double left[PHX_NRECON], right[PHX_NRECON];
+      fs[0].load(left);
+      fs[1].load(right);
+      recon_gamma1(p, left, right);
+      face_flux<MINK, 0>(p, b, xr.klo + pen / xr.nj, xr.jlo + pen % xr.nj, c, left, right);
     }
+    __syncwarp();
   }
 }
 
 template <int RECON, bool MINK>
-__global__ void __launch_bounds__(32 * X1_WARPS)
-    k_flux_x1(Par p, BView b, int mode, const __grid_constant__ CUtensorMap map, unsigned int *err) {
+__global__ void __launch_bounds__(FLUX_THREADS, flux_minb(MINK))
+    k_flux_x1(Par p, BView b, int mode, int pencils, const __grid_constant__ CUtensorMap map, unsigned int *err) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ FaceStates fs[2];
   __shared__ __align__(8) uint64_t bar;
   double *rows = reinterpret_cast<double *>(smem_raw);
   const X1Range xr = x1_range(b);
-  const int p0 = blockIdx.x * X1_PENCILS;
-  const int np = min(X1_PENCILS, xr.npencil - p0);
+  const int p0 = blockIdx.x * pencils;
+  const int np = min(pencils, xr.npencil - p0);
   if (mode != X1_LOADS && threadIdx.x == 0) {
     mbar_init(&bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   if (!x1_stage(b, xr, p0, np, mode, &map, rows, &bar, 0u, err)) return;
-  x1_compute<RECON, MINK>(p, b, xr, p0, np, rows);
+  x1_compute<RECON, MINK>(p, b, xr, p0, np, rows, fs);
 }
 
 // Batched X1: a persistent CTA walks the work list; item = (block, first
 // pencil, pencil count).  The mbarrier is reused with alternating phase.
 // maps[b] / modes[b]: block b's tensor map and staging mode.
 template <int RECON, bool MINK>
-__global__ void __launch_bounds__(32 * X1_WARPS) kb_flux_x1(Par p, const BView *views, const WorkItem *items,
-                                                            int nitems, const CUtensorMap *maps, const int *modes,
-                                                            unsigned int *err) {
+__global__ void __launch_bounds__(FLUX_THREADS, flux_minb(MINK))
+    kb_flux_x1(Par p, const BView *views, const WorkItem *items, int nitems, const CUtensorMap *maps, const int *modes,
+               unsigned int *err) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ FaceStates fs[2];
   __shared__ __align__(8) uint64_t bar;
   double *rows = reinterpret_cast<double *>(smem_raw);
   if (threadIdx.x == 0) {
@@ -277,7 +300,7 @@ __global__ void __launch_bounds__(32 * X1_WARPS) kb_flux_x1(Par p, const BView *
     if (!x1_stage(b, xr, (int)w.first, (int)(w.last - w.first), mode, maps + w.block, rows, &bar, phase, err))
       return;
     if (mode != X1_LOADS) phase ^= 1u;
-    x1_compute<RECON, MINK>(p, b, xr, (int)w.first, (int)(w.last - w.first), rows);
+    x1_compute<RECON, MINK>(p, b, xr, (int)w.first, (int)(w.last - w.first), rows, fs);
     __syncthreads();  // rows are rewritten by the next item
   }
 }
@@ -358,7 +381,7 @@ void launch_wait_probe(long long limit, unsigned int *err, cudaStream_t s) {
 // DIR 2: a = i, c = j; DIR 0 (fallback for X1): a = j, c = k.
 template <int RECON, bool MINK, int DIR>
 __device__ __forceinline__ void sweep_at(const Par &p, const BView &b, int alo, int na, int clo, int nc, int f0,
-                                         int nface, int seg, int nseg, long long t) {
+                                         int nface, int seg, int nseg, long long t, FaceStates *fs) {
   const int a = alo + (int)(t % na);
   const long long q = t / na;
   const int s = (int)(q % nseg);
@@ -393,42 +416,45 @@ __device__ __forceinline__ void sweep_at(const Par &p, const BView &b, int alo, 
   kji(fbeg - 1, k0, j0, i0);
   const double *pc = b.prim + b.idx(k0, j0, i0);  // cell fbeg-1
   const long long vs = b.vs;
-  double w[kReconLoad][5];
-#pragma unroll
-  for (int v = 0; v < kReconLoad; v++)
-#pragma unroll
-    for (int o = 0; o < 4; o++) w[v][o + 1] = pc[v * vs + (o - 2) * stride];  // cells x-2..x+1
-  double prev_ql[PHX_NRECON];
   // X2 and X3 faces of this column share X1 (= the cell centre of column a)
   FloorPt col{};
   const bool use_col = DIR != 0 && floors_x1_only(p);
   if (use_col) col = floor_point(p, b.Xc(0, a), 0.0, 0.0);
-  for (int x = fbeg - 1; x <= fend; x++) {
-    const double *pn = pc + (long long)(x - (fbeg - 1)) * stride;
-    double ql[PHX_NRECON], qr[PHX_NRECON];
-#pragma unroll
-    for (int v = 0; v < kReconLoad; v++) {
-#pragma unroll
-      for (int o = 0; o < 4; o++) w[v][o] = w[v][o + 1];
-      w[v][4] = pn[v * vs + 2 * stride];
-      recon<RECON>(w[v][0], w[v][1], w[v][2], w[v][3], w[v][4], ql[v], qr[v]);
+  // states: fs[0] and fs[1] the upper-face values of the previous and this
+  // cell in turn, fs[2] the lower-face values of this cell
+  int cur = 0;
+  for (int x = fbeg - 1; x <= fend; x++, cur ^= 1, pc += stride) {
+    const double *pn = pc;
+#pragma unroll(flux_unroll<RECON>())
+    for (int v = 0; v < kReconLoad; v++, pn += vs) {
+      double ql, qr;
+      if constexpr (RECON == PHX_RECON_WENO5Z || RECON == PHX_RECON_MP5)
+        recon<RECON>(pn[-2 * stride], pn[-stride], pn[0], pn[stride], pn[2 * stride], ql, qr);
+      else if constexpr (RECON == PHX_RECON_LINEAR)
+        recon<RECON>(0.0, pn[-stride], pn[0], pn[stride], 0.0, ql, qr);
+      else
+        recon<RECON>(0.0, 0.0, pn[0], 0.0, 0.0, ql, qr);
+      fs[cur].q[v][threadIdx.x] = ql;
+      fs[2].q[v][threadIdx.x] = qr;
     }
     if (x >= fbeg) {
       int k, j, i;
       kji(x, k, j, i);
-      recon_gamma1(p, prev_ql, qr);
-      face_flux<MINK, DIR>(p, b, k, j, i, prev_ql, qr, use_col ? &col : nullptr);
+      double left[PHX_NRECON], right[PHX_NRECON];
+      fs[cur ^ 1].load(left);
+      fs[2].load(right);
+      recon_gamma1(p, left, right);
+      face_flux<MINK, DIR>(p, b, k, j, i, left, right, use_col ? &col : nullptr);
     }
-#pragma unroll
-    for (int v = 0; v < kReconLoad; v++) prev_ql[v] = ql[v];
   }
 }
 
 template <int RECON, bool MINK, int DIR>
-__global__ void __launch_bounds__(128, PHX_SWEEP_MINB)
+__global__ void __launch_bounds__(FLUX_THREADS, flux_minb(MINK))
     k_flux_sweep(Par p, BView b, int alo, int na, int clo, int nc, int f0, int nface, int seg, int nseg) {
+  __shared__ FaceStates fs[3];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (long long)na * nc * nseg) sweep_at<RECON, MINK, DIR>(p, b, alo, na, clo, nc, f0, nface, seg, nseg, t);
+  if (t < (long long)na * nc * nseg) sweep_at<RECON, MINK, DIR>(p, b, alo, na, clo, nc, f0, nface, seg, nseg, t, fs);
 }
 
 // Sweep geometry of a block for DIR 1 (X2 faces: j in [js, je+1], i in
@@ -462,27 +488,55 @@ __host__ __device__ __forceinline__ SweepRange sweep_range(const BView &b, int d
 }
 
 template <int RECON, bool MINK, int DIR>
-__global__ void __launch_bounds__(128, PHX_SWEEP_MINB) kb_flux_sweep(Par p, const BView *views, const WorkItem *items, int nitems,
-                                                     int seg_target) {
+__global__ void __launch_bounds__(FLUX_THREADS, flux_minb(MINK))
+    kb_flux_sweep(Par p, const BView *views, const WorkItem *items, int nitems, int seg_target) {
+  __shared__ FaceStates fs[3];
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const WorkItem w = items[it];
     const long long t = w.first + threadIdx.x;
     if (t < w.last) {
       const BView &b = views[w.block];
       const SweepRange r = sweep_range(b, DIR, seg_target);
-      sweep_at<RECON, MINK, DIR>(p, b, r.alo, r.na, r.clo, r.nc, r.f0, r.nface, r.seg, r.nseg, t);
+      sweep_at<RECON, MINK, DIR>(p, b, r.alo, r.na, r.clo, r.nc, r.f0, r.nface, r.seg, r.nseg, t, fs);
     }
   }
+}
+
+// Faces per thread of a sweep over columns of nface faces.  A segment of seg
+// faces reconstructs seg + 1 cells, so long segments do less work, but a
+// launch of few long segments leaves SMs idle.  The launch takes about
+// (CTAs on the busiest SM) (seg (F + R) + R), F and R the FP64 work of a
+// face and of a cell's reconstruction; below two CTAs an SM's FP64 pipe is
+// not kept busy, so fewer count as two.  Against 32 faces throughout: 64^3 PLM
+// 1.02 -> 0.64 ms per call (69 CTAs of 33 faces before), 97 x 66 x 35 FMKS
+// WENO5-Z 1.80 -> 1.18 ms.
+static int sweep_segment(int recon, long long columns, int nface) {
+  const int nsm = sm_count();
+  const double R = recon == PHX_RECON_WENO5Z ? 1.0 : recon == PHX_RECON_MP5 ? 1.5 : 0.3;
+  int best = nface;
+  double cost = 0.0;
+  for (int seg = nface < 64 ? nface : 64; seg >= 2 || seg == nface; seg--) {
+    const long long nseg = (nface + seg - 1) / seg;
+    const long long ctas = (columns * nseg + FLUX_THREADS - 1) / FLUX_THREADS;
+    const long long busiest = (ctas + nsm - 1) / nsm;
+    const double c = (double)(busiest > 2 ? busiest : 2) * (seg * (1.0 + R) + R);
+    if (cost == 0.0 || c < cost) {
+      cost = c;
+      best = seg;
+    }
+    if (seg == 1) break;
+  }
+  return best;
 }
 
 template <int RECON, bool MINK, int DIR>
 static void launch_sweep(const Par &p, const BView &b, int alo, int na, int clo, int nc, int f0,
                          int nface, cudaStream_t s) {
-  const int target = 32;
+  const int target = sweep_segment(RECON, (long long)na * nc, nface);
   const int nseg = (nface + target - 1) / target;
   const int seg = (nface + nseg - 1) / nseg;
   const long long total = (long long)na * nc * nseg;
-  const int T = 128;
+  const int T = FLUX_THREADS;
   k_flux_sweep<RECON, MINK, DIR><<<(unsigned)((total + T - 1) / T), T, 0, s>>>(p, b, alo, na, clo, nc,
                                                                             f0, nface, seg, nseg);
 }
@@ -498,14 +552,20 @@ static void launch_fluxes_t(const Par &p, const BView &b, unsigned int *err, cud
   {
     const X1Range xr = x1_range(b);
     const int jlo = xr.jlo, nj = xr.nj, klo = xr.klo, nk = xr.npencil / xr.nj;
-    const size_t smem = (size_t)X1_PENCILS * x1_pencil_stride(b) * sizeof(double);
+    // as many pencils as leave room for the resident CTAs the registers allow
+    // (228 KB per SM, 1 KB of it per CTA); 256^3, three directions: with four
+    // pencils (two CTAs per SM) 57.6 ms, with two (four CTAs) 56.6 ms
+    const size_t pst = (size_t)x1_pencil_stride(b) * sizeof(double);
+    const size_t room = (228 * 1024) / flux_minb(MINK) - 1024 - 64 - 2 * sizeof(FaceStates);
+    const int pencils = (int)(room < pst ? 1 : (room / pst < (size_t)X1_PENCILS ? room / pst : (size_t)X1_PENCILS));
+    const size_t smem = pencils * pst;
     if (smem <= 200 * 1024) {
       auto kern = k_flux_x1<RECON, MINK>;
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       CUtensorMap map;
       memset(&map, 0, sizeof(map));
       const int mode = x1_mode(b, &map);
-      kern<<<(xr.npencil + X1_PENCILS - 1) / X1_PENCILS, 32 * X1_WARPS, smem, s>>>(p, b, mode, map, err);
+      kern<<<(xr.npencil + pencils - 1) / pencils, 32 * X1_WARPS, smem, s>>>(p, b, mode, pencils, map, err);
     } else {
       launch_sweep<RECON, MINK, 0>(p, b, jlo, nj, klo, nk, is, ie - is + 2, s);
     }

@@ -98,16 +98,20 @@ void launch_mlp_adamw(float *theta, float *grad, float *m, float *v, float lr, f
 void launch_fp64_probe(double *out, int iters, cudaStream_t s, int *nthreads_out);
 
 // ---- batched (many blocks, one persistent launch per phase; phx_batch.cu)
+inline int sm_count() {
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return nsm > 0 ? nsm : 1;
+}
 // Grid of a persistent launch: as many CTAs as fit on the GPU at once (or
 // fewer when there are fewer items); grid > 0 is taken as given.
 template <class K>
 inline int persistent_grid(K kernel, int threads, size_t smem, int nitems, int grid) {
   if (grid > 0) return grid < nitems ? grid : nitems;
-  int dev = 0, nsm = 0, occ = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem);
-  const long long g = (long long)(nsm > 0 ? nsm : 1) * (occ > 0 ? occ : 1);
+  const long long g = (long long)sm_count() * (occ > 0 ? occ : 1);
   return (int)(g < nitems ? g : nitems);
 }
 // A tiled mesh on the device (phx_mesh): per-axis global cell -> segment
