@@ -477,15 +477,6 @@ __device__ __forceinline__ double regula_falsi_warp(const Par &p, Residual &res,
 // 3.90 -> 1.15 ms (7.0 -> 1.0 evaluations), 1000 cold zones 96 -> 40 us; the
 // root's error against the sampled state 3e-14 -> 5e-15.
 
-// a > b for doubles by their bit patterns (no NaN; -0 sorts below +0): an FP64
-// comparison holds the FP64 pipe like an FMA.
-__device__ __forceinline__ bool gt_bits(double a, double b) {
-  long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-  x ^= (x >> 63) & 0x7fffffffffffffffll;
-  y ^= (y >> 63) & 0x7fffffffffffffffll;
-  return x > y;
-}
-
 // float from a double by bit operations (a conversion instruction holds the
 // FP64 pipe): truncated, 0 below and +-max above the FP32 normal range.
 __device__ __forceinline__ float d2f_bits(double x) {

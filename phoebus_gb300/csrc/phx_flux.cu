@@ -52,17 +52,54 @@ __device__ __forceinline__ void face_flux(const Par &p, const BView &b, int k, i
     f.fl = floor_point(p, DIR == 0 ? b.Xf(0, i) : b.Xc(0, i), DIR == 1 ? b.Xf(1, j) : b.Xc(1, j),
                        DIR == 2 ? b.Xf(2, k) : b.Xc(2, k));
   }
-  const double gam_max = p.g0, sie_max = p.smax0;
-  double Ul[PHX_NCONS], Fl[PHX_NCONS], Ur[PHX_NCONS], Fr[PHX_NCONS];
-  double vml, vpl, vmr, vpr;
-  prim_to_flux<MINK, DIR>(p, f, ql, vml, vpl, Ul, Fl, sie_max, gam_max);
-  prim_to_flux<MINK, DIR>(p, f, qr, vmr, vpr, Ur, Fr, sie_max, gam_max);
   const double gdet = MINK ? 1.0 : f.gdet;
   const double gammadet = MINK ? 1.0 : f.gammadet;
   const long long id = b.idx(k, j, i);
   double *fx = b.flux + (long long)DIR * PHX_NCONS * b.vs + id;
   const int ncons = p.mhd ? PHX_NCONS : 5;
   double sig;
+#ifndef PHX_EXACT
+  // both solvers as F = cl F_l + cr F_r + c (U_r - U_l), with the states'
+  // F = U vtil + G collected by U
+  FluxState l, r;
+  flux_state<MINK, DIR>(p, f, ql, l);
+  flux_state<MINK, DIR>(p, f, qr, r);
+  double kl, kr, kc;
+  if (p.riemann == PHX_RIEMANN_LLF) {
+    sig = max_num(max_num(-l.vm, l.vp), max_num(-r.vm, r.vp));
+    kl = kr = 0.5 * gdet;
+    kc = -0.5 * sig * gammadet;
+  } else {
+    const double cl = min_num(min_num(l.vm, r.vm), 0.0);
+    const double cr = max_num(max_num(l.vp, r.vp), 0.0);
+    const double dc = cr - cl;
+    const int e = dexp(dc);
+    const double idc = (e >= 16 && e <= 2030) ? rcp_nr(dc) : ratio_p(1.0, dc);
+    const double gi = gdet * idc;
+    kl = cr * gi;
+    kr = -cl * gi;
+    kc = cr * cl * (MINK ? idc : gammadet * idc);
+    sig = max_num(-cl, cr);
+  }
+  const double al = fma(kl, l.vtil, -kc), ar = fma(kr, r.vtil, kc);
+#pragma unroll
+  for (int m = 0; m < PHX_NCONS; m++) {
+    if (m >= ncons) continue;
+    double F;
+    if (m == PHX_CRHO)
+      F = fma(al, l.U[m], ar * r.U[m]);
+    else if (m == PHX_CB + DIR)  // B^d v^d - B^d v^d is 0 in both states
+      F = kc * (r.U[m] - l.U[m]);
+    else
+      F = fma(al, l.U[m], fma(ar, r.U[m], fma(kl, l.G[m], kr * r.G[m])));
+    fx[m * b.vs] = F;
+  }
+#else
+  const double gam_max = p.g0, sie_max = p.smax0;
+  double Ul[PHX_NCONS], Fl[PHX_NCONS], Ur[PHX_NCONS], Fr[PHX_NCONS];
+  double vml, vpl, vmr, vpr;
+  prim_to_flux<MINK, DIR>(p, f, ql, vml, vpl, Ul, Fl, sie_max, gam_max);
+  prim_to_flux<MINK, DIR>(p, f, qr, vmr, vpr, Ur, Fr, sie_max, gam_max);
   if (p.riemann == PHX_RIEMANN_LLF) {
     const double cmax = rmax(rmax(-vml, vpl), rmax(-vmr, vpr));
 #pragma unroll
@@ -73,21 +110,14 @@ __device__ __forceinline__ void face_flux(const Par &p, const BView &b, int k, i
     const double cl = rmin(rmin(vml, vmr), 0.0);
     const double cr = rmax(rmax(vpl, vpr), 0.0);
     const double crcl = cr * cl;
-    const double inv_cr_cl = ratio_p(1.0, cr - cl);
-#ifdef PHX_EXACT
+    const double inv_cr_cl = ratio(1.0, cr - cl);
 #pragma unroll
     for (int m = 0; m < PHX_NCONS; m++)
       if (m < ncons)
         fx[m * b.vs] = ((cr * Fl[m] - cl * Fr[m]) * gdet + crcl * (Ur[m] - Ul[m]) * gammadet) * inv_cr_cl;
-#else
-    // the per-face factors formed once: F_l cr' - F_r cl' + (U_r - U_l) c'
-    const double crg = cr * gdet * inv_cr_cl, clg = cl * gdet * inv_cr_cl, cc = crcl * gammadet * inv_cr_cl;
-#pragma unroll
-    for (int m = 0; m < PHX_NCONS; m++)
-      if (m < ncons) fx[m * b.vs] = fma(crg, Fl[m], fma(-clg, Fr[m], cc * (Ur[m] - Ul[m])));
-#endif
     sig = rmax(-cl, cr);
   }
+#endif
   b.face_sig[(long long)DIR * b.vs + id] = sig;
 }
 
