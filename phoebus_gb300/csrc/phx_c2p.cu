@@ -116,7 +116,12 @@ void launch_p2c_zones(const Par &p, long long n, const double *prim, const doubl
 // network out of the root-find kernel keeps that kernel's instruction
 // footprint small (fused, the two codes thrashed the instruction cache).
 constexpr int C2P_THREADS = 128;
-constexpr int C2P_WARPS = C2P_THREADS / 32;
+// Resident CTAs per SM the root-find kernels' registers are bounded for.
+#ifdef PHX_EXACT
+constexpr int c2p_minb(bool) { return 1; }
+#else
+constexpr int c2p_minb(bool mink) { return mink ? 4 : 3; }
+#endif
 
 // Zones of a block index box.
 struct BoxZones {
@@ -347,7 +352,7 @@ __device__ __forceinline__ void rf_unpack(unsigned long long w, RFState &s) {
 // and left to k_c2p_retry, so that one slow zone does not hold 31 finished
 // lanes of its warp.
 template <class Z, bool MINK, bool LEARNED>
-__global__ void __launch_bounds__(C2P_THREADS) k_c2p(Par p, Z zones, long long t0, long long count,
+__global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK)) k_c2p(Par p, Z zones, long long t0, long long count,
                                                       const double *brk, int cap, RetryBuf rb, DevStats *stats,
                                                       unsigned int *err) {
   __shared__ unsigned int s_hist[PHX_C2P_HIST];
@@ -613,7 +618,7 @@ __global__ void __launch_bounds__(C2P_THREADS) kb_mlp_bracket(Par p, const BView
 // so warm zones (all of them once a run is under way) go through exactly the
 // plain kernel's code.
 template <bool MINK, bool LEARNED>
-__global__ void __launch_bounds__(C2P_THREADS) kb_c2p(Par p, const BView *views, const WorkItem *items, int nitems,
+__global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK)) kb_c2p(Par p, const BView *views, const WorkItem *items, int nitems,
                                                        double *brk, DevStats *stats, unsigned int *err, int only) {
   if (only == 2 && *reinterpret_cast<const unsigned long long *>(brk + 4 * (long long)nitems * C2P_THREADS) == 0)
     return;  // no cold zone

@@ -37,7 +37,7 @@ struct Residual {
   }
   __device__ __forceinline__ double vhatsq_mu(double mu, double rbarsq) {
     const double vsq_trial = mu * mu * rbarsq;
-    if (vsq_trial > v0sq) {
+    if (gt(vsq_trial, v0sq)) {
       used_gamma_max = true;
       return v0sq;
     }
@@ -47,7 +47,7 @@ struct Residual {
   __device__ __forceinline__ double iWhat_mu(double vhatsq) const { return sqrt(1.0 - vhatsq); }
   __device__ __forceinline__ double rhohat_mu(double iWhat) {
     const double rho_trial = D * iWhat;
-    if (rho_trial <= rho_floor) {
+    if (!gt(rho_trial, rho_floor) && !is_nan(rho_trial)) {
       used_density_floor = true;
       return rho_floor;
     }
@@ -63,34 +63,36 @@ struct Residual {
     const double ehat_trial = What * (qbar - mu * rbarsq) + vhatsq * What * ratio_p(What, 1.0 + What);
     used_energy_floor = false;
     used_energy_max = false;
-    if (ehat_trial <= e_floor) {
+    if (!gt(ehat_trial, e_floor) && !is_nan(ehat_trial)) {
       used_energy_floor = true;
       return e_floor;
-    } else if (ehat_trial > e_max) {
+    } else if (gt(ehat_trial, e_max)) {
       used_energy_max = true;
       return e_max;
     }
     return ehat_trial;
   }
-  // ehat_mu with the density from a known 1/W (production build)
-  __device__ __forceinline__ double ehat_mu_iw(const Par &p, double mu, double qbar, double rbarsq, double vhatsq,
-                                               double What, double iWhat) {
-    double rho = rhohat_mu(iWhat);
+  // the energy bounds of ehat_mu at density rho (production build)
+  __device__ __forceinline__ double bound_ehat(const Par &p, double rho, double ehat_trial) {
     double e_floor;
     floors_from(p, fl, rho, e_floor);
     e_floor *= p.fsf;
-    // What = 1 / sqrt(1 - vhatsq): vhatsq What^2 / (1 + What) = What - 1
-    const double ehat_trial = fma(What, qbar - mu * rbarsq, What - 1.0);
     used_energy_floor = false;
     used_energy_max = false;
-    if (ehat_trial <= e_floor) {
+    if (!gt(ehat_trial, e_floor) && !is_nan(ehat_trial)) {
       used_energy_floor = true;
       return e_floor;
-    } else if (ehat_trial > e_max) {
+    } else if (gt(ehat_trial, e_max)) {
       used_energy_max = true;
       return e_max;
     }
     return ehat_trial;
+  }
+  // ehat_mu with the density from a known 1/W (production build);
+  // What = 1 / sqrt(1 - vhatsq): vhatsq What^2 / (1 + What) = What - 1
+  __device__ __forceinline__ double ehat_mu_iw(const Par &p, double mu, double qbar, double rbarsq, double vhatsq,
+                                               double What, double iWhat) {
+    return bound_ehat(p, rhohat_mu(iWhat), fma(What, qbar - mu * rbarsq, What - 1.0));
   }
   __device__ __forceinline__ double operator()(const Par &p, double mu) {
     const double x = x_mu(mu);
@@ -145,8 +147,7 @@ __device__ __forceinline__ bool c2p_setup(const Par &p, const Pt &g, const doubl
                                           double x1, double x2, double x3, Residual &res,
                                           double rcon[3], double rcov[3], double bu[3],
                                           double Bprim[3], double &bdotr) {
-  const int num_nans = isnan(U[PHX_CRHO]) + isnan(U[PHX_CMOM]) + isnan(U[PHX_CENG]);
-  if (num_nans > 0) return false;
+  if (is_nan(U[PHX_CRHO]) || is_nan(U[PHX_CMOM]) || is_nan(U[PHX_CENG])) return false;
   const double gdet = MINK ? 1.0 : g.detgam;
   const double igdet = MINK ? 1.0 : rcp_p(gdet);  // 1 / 1 = 1 in both builds
   double rhoflr = 0.0, epsflr;
@@ -201,7 +202,7 @@ __device__ __forceinline__ bool c2p_setup(const Par &p, const Pt &g, const doubl
       bdotr += bu[ii] * rcov[ii];
     }
     bsq = dot_sp<MINK>(g, bu, bu);
-    bsq = fmax(0.0, bsq);
+    bsq = clamp0(bsq);
     rbsq = bdotr * bdotr;
     bsq_rpsq = bsq * rsq - rbsq;
   }
@@ -471,11 +472,13 @@ __device__ __forceinline__ double regula_falsi_warp(const Par &p, Residual &res,
 // follow).  A zone that does not pass these tests (floors or caps switching
 // at the root, values outside the FP32 range, NaN) takes the reference's
 // bracketed iteration instead.
-// Measured against the bracketed iteration in FP64 (GB300): 1.2e7 cold
-// Kerr-Schild zones at tolerance 1e-13 30.0 -> 7.4 ms (12.8 -> 1.05 FP64
-// residual evaluations per zone), a 136^3 Minkowski block from stale mu
-// 3.90 -> 1.15 ms (7.0 -> 1.0 evaluations), 1000 cold zones 96 -> 40 us; the
-// root's error against the sampled state 3e-14 -> 5e-15.
+// Measured against the bracketed iteration in FP64 (GB300, with the reciprocals
+// on the integer pipe and c2p_finish's algebra): 1.2e7 cold Kerr-Schild zones
+// at tolerance 1e-13 30.0 -> 5.6 ms (12.8 -> 1.05 FP64 residual evaluations per
+// zone), a 136^3 Minkowski block from stale mu 3.90 -> 0.87 ms (7.0 -> 1.0
+// evaluations; 147 FP64 instructions per zone, the FP64 pipe busy 94% of the
+// time), 1000 cold zones 96 -> 40 us; the root's error against the sampled
+// state 3e-14 -> 5e-15.
 
 // float from a double by bit operations (a conversion instruction holds the
 // FP64 pipe): truncated, 0 below and +-max above the FP32 normal range.
@@ -725,49 +728,54 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
     last = d;
   }
   if (!(s > 1e-3f && m > 1e-12f && m <= 1.0f)) return false;
+  // float-pair Newton steps until the step is at the pairs' rounding; the slope
+  // follows the secant (the residual's branches differ in slope at the root)
   FF mp = {m, 0.0f};
-  float is = rcp_f32(s);
-  float fp = rf.evalp(mp);
+  float is = rcp_f32(s), step = 0.0f, fp = 0.0f;
 #pragma unroll 1
-  for (int it = 0; it < 2; it++) {
-    const float step = fp * is;
+  for (int it = 0; it < 5; it++) {
+    const float f = rf.evalp(mp);
+    if (it > 0 && fabsf(step) > 1e-7f * m) is = step * rcp_f32(fp - f);
+    step = f * is;
+    fp = f;
     if (!(fabsf(step) <= 0.5f * m)) return false;
-    const FF mn = ff_addf(mp, -step);
-    const float fn = it == 0 ? rf.evalp(mn) : 0.0f;
-    if (it == 0 && fabsf(step) > 1e-5f * m) is = step * rcp_f32(fp - fn);
-    mp = mn;
-    fp = fn;
+    mp = ff_addf(mp, -step);
+    if (fabsf(step) <= 4e-12f * m) break;
   }
-  double x = f2d_bits(mp.h) + f2d_bits(mp.l), fx;
+  if (!(is > 0.0f && is < 1e3f)) return false;
+  double x = f2d_bits(mp.h) + f2d_bits(mp.l);
   const float tol = d2f_bits(p.c2p_tol);
-  if (!(is > 0.0f && x > 0.0 && x <= 1.0) || !rf.eval64(p, res, x, fx)) return false;
-  float f = d2f_bits(fx);
-  out.iterations = 0;
-  out.evals = 1;
-  // the slope is good to a few parts in 1e3 where a secant confirmed it
-  float gain = 1.0f;
+  float f = 0.0f, gain = 1.0f;
+  out.iterations = out.evals = 0;
+#pragma unroll 1
   for (;;) {
-    const float step = f * is;
-    const float as = fabsf(step);
-    const double xn = x - f2d_bits(step);
-    out.iterations++;
-    if (!(as <= 0.5f * m)) return false;
-    if (as <= gain * tol) {  // the error after this step: the step times the slope's relative error
-      mu = xn < 1.0 ? xn : 1.0;
-      return xn > 0.0;
-    }
-    if (out.evals >= C2P_FAST_EVALS || !(xn > 0.0 && xn <= 1.0) || !rf.eval64(p, res, xn, fx)) return false;
-    const float fn = d2f_bits(fx);
-    out.evals++;
-    if (as > 1e-9f * m) {
+    double f64;
+    if (out.evals >= C2P_FAST_EVALS || !(x > 0.0 && x <= 1.0) || !rf.eval64(p, res, x, f64)) return false;
+    const float fn = d2f_bits(f64);
+    if (out.evals > 0 && fabsf(step) > 1e-9f * m) {  // secant through the last two evaluations
       const float isec = step * rcp_f32(f - fn);
       if (!(isec > 0.0f && isec < 1e3f)) return false;
       gain = fabsf(is * rcp_f32(isec) - 1.0f) <= 0.03125f ? 16.0f : 1.0f;
       is = isec;
     }
-    x = xn;
+    out.evals++;
+    out.iterations++;
     f = fn;
+    step = f * is;
+    if (!(fabsf(step) <= 0.5f * m)) return false;
+    x -= f2d_bits(step);
+    // the error after this step: the step times the slope's relative error
+    if (fabsf(step) <= gain * tol) {
+      mu = x < 1.0 ? x : 1.0;
+      return x > 0.0;
+    }
   }
+}
+
+// The reference's iteration for the zones the fast root leaves, kept out of
+// the callers' instruction stream.
+static __device__ __noinline__ double c2p_slow_root(const Par &p, Residual res, bool need, double guess, C2POut *out) {
+  return regula_falsi_warp<false>(p, res, need, 0.0, 1.0, guess, *out);
 }
 #endif
 
@@ -782,7 +790,7 @@ __device__ __forceinline__ double c2p_root_warp(const Par &p, Residual &res, boo
   if (valid && c2p_fast_allowed(p)) need = !c2p_fast_root<LEARNED>(p, res, guess, lb, mu, out);
   if (!__any_sync(0xffffffffu, need)) return mu;
   C2POut slow{0, 0, false, true, false, false};
-  const double ms = regula_falsi_warp<false>(p, res, need, 0.0, 1.0, guess, slow);
+  const double ms = c2p_slow_root(p, res, need, guess, &slow);
   if (need) {
     out.iterations = slow.iterations;
     out.evals = slow.evals;
@@ -806,43 +814,58 @@ __device__ __forceinline__ void c2p_finish(const Par &p, const Pt &g, Residual &
                                            double prim[PHX_NPRIM], double U[PHX_NCONS],
                                            double sig[3], bool &used_bounds_out) {
   prim[PHX_PMU] = mu;
+#ifndef PHX_EXACT
+  // production build: the residual's algebra (FastResidual), W and 1/W from
+  // one reciprocal square root, P = gm1 rho e, the three-velocity before W v
+  const double x = rcp_p(fma(mu, res.bsq, 1.0));
+  const double mr = mu * res.rbsq, mux = mu * x;
+  const double mrb = mu * (x * fma(x, res.rsq + mr, mr));
+  double vsq = mu * mrb;
+  res.used_gamma_max = gt(vsq, res.v0sq);
+  if (res.used_gamma_max) vsq = res.v0sq;
+  const double om = 1.0 - vsq;
+  const double W = rsqrt_p(om), iW = om * W;
+  prim[PHX_PRHO] = res.rhohat_mu(iW);
+  const double A = fma(-0.5 * res.bsq_rpsq, mux * mux, fma(-0.5, res.bsq, res.q)) - mrb;
+  double eng = res.bound_ehat(p, prim[PHX_PRHO], fma(W, A, W - 1.0));
+  prim[PHX_PTMP] = eos_T_rho_sie(p, prim[PHX_PRHO], eng);
+  eng *= prim[PHX_PRHO];
+  prim[PHX_PENG] = eng;
+  prim[PHX_PPRS] = clamp0(p.gm1 * eng);
+  // bmod / P of the ideal gas is Gamma wherever P > 0 (the quotient, NaN for
+  // P = 0, elsewhere)
+  prim[PHX_PGM1] = __double_as_longlong(prim[PHX_PPRS]) > 0
+                       ? p.gm1 + 1.0
+                       : div_p(eos_bmod_rho_T(p, prim[PHX_PRHO], prim[PHX_PTMP]), prim[PHX_PPRS]);
+  double v3[3], vel[3];
+  const double mbr = mu * bdotr;
+#pragma unroll
+  for (int ii = 0; ii < 3; ii++) {
+    v3[ii] = mux * fma(mbr, bu_in[ii], rcon[ii]);
+    vel[ii] = W * v3[ii];
+    prim[PHX_PVEL + ii] = vel[ii];
+  }
+#else
   const double x = res.x_mu(mu);
   const double rbarsq = res.rbarsq_mu(mu, x);
   const double vsq = res.vhatsq_mu(mu, rbarsq);
-#ifdef PHX_EXACT
   const double iW = res.iWhat_mu(vsq);
   const double W = rcp_p(iW);
-#else
-  // W and 1/W from one reciprocal square root, as in the residual
-  const double W = rsqrt_p(1.0 - vsq);
-  const double iW = (1.0 - vsq) * W;
-#endif
   prim[PHX_PRHO] = res.rhohat_mu(iW);
   const double qbar = res.qbar_mu(mu, x);
-#ifdef PHX_EXACT
   double eng = res.ehat_mu(p, mu, qbar, rbarsq, vsq, W);
-#else
-  double eng = res.ehat_mu_iw(p, mu, qbar, rbarsq, vsq, W, iW);  // 1/W known
-#endif
   prim[PHX_PTMP] = eos_T_rho_sie(p, prim[PHX_PRHO], eng);
   eng *= prim[PHX_PRHO];
   prim[PHX_PENG] = eng;
   prim[PHX_PPRS] = eos_P_rho_T(p, prim[PHX_PRHO], prim[PHX_PTMP]);
-#ifdef PHX_EXACT
   prim[PHX_PGM1] = div_p(eos_bmod_rho_T(p, prim[PHX_PRHO], prim[PHX_PTMP]), prim[PHX_PPRS]);
-#else
-  // production build: bmod / P of the ideal gas is Gamma wherever P > 0 (the
-  // quotient, NaN for P = 0, elsewhere)
-  prim[PHX_PGM1] = prim[PHX_PPRS] > 0.0
-                       ? p.gm1 + 1.0
-                       : div_p(eos_bmod_rho_T(p, prim[PHX_PRHO], prim[PHX_PTMP]), prim[PHX_PPRS]);
-#endif
   double vel[3];
 #pragma unroll
   for (int ii = 0; ii < 3; ii++) {
     vel[ii] = W * mu * x * (rcon[ii] + mu * bdotr * bu_in[ii]);
     prim[PHX_PVEL + ii] = vel[ii];
   }
+#endif
   double bu[3] = {0.0, 0.0, 0.0};
   if (p.mhd) {
 #pragma unroll
@@ -862,8 +885,13 @@ __device__ __forceinline__ void c2p_finish(const Par &p, const Pt &g, Residual &
 #pragma unroll
     for (int ii = 0; ii < 3; ii++) U[PHX_CMOM + ii] = S[ii];
   } else {
+#ifdef PHX_EXACT
 #pragma unroll
     for (int m = 0; m < 3; m++) vel[m] *= iW;
+#else
+#pragma unroll
+    for (int m = 0; m < 3; m++) vel[m] = v3[m];
+#endif
     double bsq = 0.0;
     if (p.mhd) {
       double bdotv;

@@ -24,23 +24,70 @@ constexpr double kSMALL = 10 * 2.2250738585072014e-308;  // 10 * DBL_MIN
 constexpr double kEPS = 10 * 2.220446049250313e-16;      // 10 * DBL_EPSILON
 constexpr double kDBLMAX = 1.7976931348623157e308;
 
+// Comparisons of doubles on the integer pipe (an FP64 comparison holds the
+// FP64 pipe like an FMA): order_bits is increasing in x (-0 below +0, NaN
+// with a clear sign bit on top).  max_num / min_num return the other operand
+// where one is NaN, as fmax / fmin do.
+__device__ __forceinline__ long long order_bits(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double from_order_bits(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+__device__ __forceinline__ bool gt_bits(double a, double b) { return order_bits(a) > order_bits(b); }
+__device__ __forceinline__ bool nan_bits(double x) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ double max_num(double a, double b) {
+  return nan_bits(a) || (gt_bits(b, a) && !nan_bits(b)) ? b : a;
+}
+__device__ __forceinline__ double min_num(double a, double b) {
+  return nan_bits(a) || (gt_bits(a, b) && !nan_bits(b)) ? b : a;
+}
+
 // std::max / std::min as the reference calls them: the first argument comes
 // back when the comparison is false, so a NaN there propagates (fmax / fmin
 // would drop it).  The exact build keeps that for bit-for-bit parity on
-// every input, NaN states included; the production build uses the one-
-// instruction fmax / fmin (the two differ only where an argument is NaN).
+// every input, NaN states included; the production build uses max_num /
+// min_num (the two differ only where an argument is NaN, or for zeros of
+// different sign).
 __device__ __forceinline__ double rmax(double a, double b) {
 #ifdef PHX_EXACT
   return (a < b) ? b : a;
 #else
-  return fmax(a, b);
+  return max_num(a, b);
 #endif
 }
 __device__ __forceinline__ double rmin(double a, double b) {
 #ifdef PHX_EXACT
   return (b < a) ? b : a;
 #else
-  return fmin(a, b);
+  return min_num(a, b);
+#endif
+}
+// fmax(0, x)
+__device__ __forceinline__ double clamp0(double x) {
+#ifdef PHX_EXACT
+  return fmax(0.0, x);
+#else
+  const long long b = __double_as_longlong(x);
+  return b <= 0x7ff0000000000000ll && b > 0 ? x : 0.0;
+#endif
+}
+// a > b (false where either is NaN)
+__device__ __forceinline__ bool gt(double a, double b) {
+#ifdef PHX_EXACT
+  return a > b;
+#else
+  return gt_bits(a, b) && !nan_bits(a) && !nan_bits(b);
+#endif
+}
+__device__ __forceinline__ bool is_nan(double x) {
+#ifdef PHX_EXACT
+  return isnan(x);
+#else
+  return nan_bits(x);
 #endif
 }
 __device__ __forceinline__ double make_positive(double v) { return rmax(v, kEPS); }
@@ -84,28 +131,6 @@ __device__ __forceinline__ double rcp_nr(double x) {
 }
 // biased exponent of a double, on the integer pipe
 __device__ __forceinline__ int dexp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
-
-// Comparisons of doubles on the integer pipe (an FP64 comparison holds the
-// FP64 pipe like an FMA): order_bits is increasing in x (-0 below +0, NaN
-// with a clear sign bit on top).  max_num / min_num return the other operand
-// where one is NaN, as fmax / fmin do.
-__device__ __forceinline__ long long order_bits(double x) {
-  const long long b = __double_as_longlong(x);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
-}
-__device__ __forceinline__ double from_order_bits(long long k) {
-  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
-}
-__device__ __forceinline__ bool gt_bits(double a, double b) { return order_bits(a) > order_bits(b); }
-__device__ __forceinline__ bool nan_bits(double x) {
-  return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
-}
-__device__ __forceinline__ double max_num(double a, double b) {
-  return nan_bits(a) || (gt_bits(b, a) && !nan_bits(b)) ? b : a;
-}
-__device__ __forceinline__ double min_num(double a, double b) {
-  return nan_bits(a) || (gt_bits(a, b) && !nan_bits(b)) ? b : a;
-}
 
 // 1/x for the production build (IEEE division in the exact build); falls back
 // to the division when x is outside the normal range the Newton form handles.
@@ -165,6 +190,8 @@ __device__ __forceinline__ double ratio_p(double a, double b) {
 #ifdef PHX_EXACT
   return ratio(a, b);
 #else
+  const int e = dexp(b);  // kSMALL is below half an ulp of b from an exponent of -960 on
+  if (e >= 64 && e <= 2030) return a * rcp_nr(b);
   const double sgn = b >= 0 ? 1.0 : -1.0;
   return a * rcp_p(b + sgn * kSMALL);
 #endif
@@ -218,23 +245,23 @@ __device__ __forceinline__ void recon_gamma1(const Par &p, double *ql, double *q
 
 // ------------------------------------------------ singularity-eos IdealGas
 __device__ __forceinline__ double eos_P_rho_sie(const Par &p, double rho, double sie) {
-  return fmax(0.0, p.gm1 * rho * sie);
+  return clamp0(p.gm1 * rho * sie);
 }
 __device__ __forceinline__ double eos_T_rho_sie(const Par &p, double rho, double sie) {
 #ifdef PHX_EXACT
-  return fmax(0.0, div_p(sie, p.Cv));
+  return clamp0(div_p(sie, p.Cv));
 #else
-  return fmax(0.0, sie * p.iCv);  // production build: the host's 1/Cv
+  return clamp0(sie * p.iCv);  // production build: the host's 1/Cv
 #endif
 }
 __device__ __forceinline__ double eos_P_rho_T(const Par &p, double rho, double T) {
-  return fmax(0.0, p.gm1 * rho * p.Cv * T);
+  return clamp0(p.gm1 * rho * p.Cv * T);
 }
 __device__ __forceinline__ double eos_bmod_rho_T(const Par &p, double rho, double T) {
-  return fmax(0.0, (p.gm1 + 1) * p.gm1 * rho * p.Cv * T);
+  return clamp0((p.gm1 + 1) * p.gm1 * rho * p.Cv * T);
 }
 __device__ __forceinline__ double eos_bmod_rho_sie(const Par &p, double rho, double sie) {
-  return fmax(0.0, p.gm1 * (p.gm1 + 1) * rho * sie);
+  return clamp0(p.gm1 * (p.gm1 + 1) * rho * sie);
 }
 
 // ------------------------------------------------------- fixup.hpp Bounds
@@ -447,21 +474,14 @@ __device__ __forceinline__ void signal_speeds(double rho, double u, double p, do
     cssq = div_p(gam1 * p, rho_rel);
   }
 #endif
+#ifdef PHX_EXACT
   cssq += vasq - cssq * vasq;
   const double alpha = MINK ? 1.0 : g.alpha;
   const double vcoff = div_p(alpha, 1.0 - vsq * cssq);
 #pragma unroll
   for (int m = 0; m < 3; m++) {
     const double gmm = MINK ? 1.0 : g.gamcon[m][m];
-#ifdef PHX_EXACT
     const double vpm = sqrt(cssq * (1.0 - vsq) * (gmm * (1.0 - vsq * cssq) - v[m] * v[m] * (1.0 - cssq)));
-#else
-    // production build: sqrt(x) as x rsqrt(x) for normal x > 0 (zero, negative
-    // and extreme arguments take the IEEE square root)
-    const double vpm_sq = cssq * (1.0 - vsq) * (gmm * (1.0 - vsq * cssq) - v[m] * v[m] * (1.0 - cssq));
-    const int ev = dexp(vpm_sq);
-    const double vpm = (vpm_sq > 0.0 && ev >= 16 && ev <= 2030) ? vpm_sq * rsqrt_nr(vpm_sq) : sqrt(vpm_sq);
-#endif
     double vp = vcoff * (v[m] * (1.0 - cssq) + vpm);
     double vm = vcoff * (v[m] * (1.0 - cssq) - vpm);
     if constexpr (!MINK) {
@@ -470,6 +490,23 @@ __device__ __forceinline__ void signal_speeds(double rho, double u, double p, do
     }
     sig[m] = rmax(fabs(vp), fabs(vm));
   }
+#else
+  // production build: max(|a + e|, |a - e|) = |a| + e with a = c v (1 - cs^2) - beta
+  // and e = c sqrt(...) >= 0; sqrt(x) as x rsqrt(x) for normal x > 0 (zero,
+  // negative and extreme arguments take the IEEE square root)
+  cssq = fma(vasq, 1.0 - cssq, cssq);
+  const double c1 = 1.0 - cssq, Q = fma(-vsq, cssq, 1.0), k = cssq * (1.0 - vsq);
+  const double vcoff = MINK ? rcp_p(Q) : g.alpha * rcp_p(Q);
+#pragma unroll
+  for (int m = 0; m < 3; m++) {
+    const double t = v[m] * c1;
+    const double rad = k * fma(-v[m], t, MINK ? Q : g.gamcon[m][m] * Q);
+    const int ev = __double2hiint(rad) >> 20;  // biased exponent, negative for rad < 0
+    const double vpm = (ev >= 16 && ev <= 2030) ? rad * rsqrt_nr(rad) : sqrt(rad);
+    const double a = MINK ? vcoff * t : fma(vcoff, t, -g.beta[m]);
+    sig[m] = fma(vcoff, vpm, fabs(a));
+  }
+#endif
 }
 
 // p2c (prim2con.hpp:48-102)
