@@ -1084,7 +1084,7 @@ __device__ __forceinline__ void prim_to_flux(const Par &par, const Face &f, cons
 // state instead of once per variable, comparisons on the integer pipe, and
 // the lowered vectors shared between the contractions.  About 70 FP64
 // instructions on Minkowski (82 and 16 FP64 comparisons in prim_to_flux):
-// 256^3 WENO5-Z fluxes 56.6 -> 53.5 ms, 64^3 PLM 0.64 -> 0.53 ms (with
+// 256^3 WENO5-Z fluxes 56.6 -> 54.9 ms, 64^3 PLM 0.64 -> 0.56 ms (with
 // recon_plm_fast).
 struct FluxState {
   double U[PHX_NCONS], G[PHX_NCONS], vtil, vm, vp;

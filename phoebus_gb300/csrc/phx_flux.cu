@@ -59,8 +59,8 @@ __device__ __forceinline__ void face_flux(const Par &p, const BView &b, int k, i
   const int ncons = p.mhd ? PHX_NCONS : 5;
   double sig;
 #ifndef PHX_EXACT
-  // both solvers as F = cl F_l + cr F_r + c (U_r - U_l), with the states'
-  // F = U vtil + G collected by U
+  // both solvers as F = kl F_l + kr F_r + kc (U_r - U_l), with the states'
+  // F = U vtil + G
   FluxState l, r;
   flux_state<MINK, DIR>(p, f, ql, l);
   flux_state<MINK, DIR>(p, f, qr, r);
@@ -81,17 +81,16 @@ __device__ __forceinline__ void face_flux(const Par &p, const BView &b, int k, i
     kc = cr * cl * (MINK ? idc : gammadet * idc);
     sig = max_num(-cl, cr);
   }
-  const double al = fma(kl, l.vtil, -kc), ar = fma(kr, r.vtil, kc);
+  // U_r - U_l formed first: equal states then carry no rounding of c U
+  const double al = kl * l.vtil, ar = kr * r.vtil;
 #pragma unroll
   for (int m = 0; m < PHX_NCONS; m++) {
     if (m >= ncons) continue;
-    double F;
-    if (m == PHX_CRHO)
-      F = fma(al, l.U[m], ar * r.U[m]);
-    else if (m == PHX_CB + DIR)  // B^d v^d - B^d v^d is 0 in both states
-      F = kc * (r.U[m] - l.U[m]);
-    else
-      F = fma(al, l.U[m], fma(ar, r.U[m], fma(kl, l.G[m], kr * r.G[m])));
+    double F = kc * (r.U[m] - l.U[m]);
+    if (m != PHX_CB + DIR) {  // B^d v^d - B^d v^d is 0 in both states
+      F = fma(al, l.U[m], fma(ar, r.U[m], F));
+      if (m != PHX_CRHO) F = fma(kl, l.G[m], fma(kr, r.G[m], F));
+    }
     fx[m * b.vs] = F;
   }
 #else
