@@ -18,6 +18,7 @@
 // (fluxes).  The fluxes of a face need only the row d of the pressure
 // tensors P^i_j of its direction; the other rows are not formed.
 #include <cfloat>
+#include <type_traits>
 
 #include "phx_m1.cuh"
 
@@ -35,10 +36,20 @@ namespace rad {
 #define DW(x) ((x) * iW)
 #endif
 
-// std::min / std::max (NaN handling of the reference)
-__device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
-__device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
+// std::min / std::max (NaN handling of the reference); the production build
+// compares on the integer pipe
+__device__ __forceinline__ double smin(double a, double b) { return gt(a, b) ? b : a; }
+__device__ __forceinline__ double smax(double a, double b) { return gt(b, a) ? b : a; }
 __device__ __forceinline__ double sgn(double v) { return (double)((0.0 <= v) - (v < 0.0)); }
+// sqrt(x): the production build's x rsqrt(x) for normal x > 0
+__device__ __forceinline__ double sqrt_p(double x) {
+#ifdef PHX_EXACT
+  return sqrt(x);
+#else
+  const int e = __double2hiint(x) >> 20;  // biased exponent, negative for x < 0
+  return (e >= 16 && e <= 2030) ? x * rsqrt_nr(x) : sqrt(x);
+#endif
+}
 
 // tanh: e^y by Cody-Waite reduction y = n ln2 + r (32-bit head of ln2, so
 // n * head is exact) and the Taylor series of e^r to degree 13; e^y - 1 by its
@@ -94,7 +105,7 @@ __device__ __forceinline__ double tanh_r(double x) {
   } else {
     const double y = -2.0 * ax;
     const double m = (y > -0.25) ? expm1_small(y) : exp_neg(y) - 1.0;
-    t = -m / (2.0 + m);
+    t = div_p(-m, 2.0 + m);
   }
   return copysign(t, x);
 }
@@ -123,7 +134,7 @@ __device__ __forceinline__ double lorentz3(const double vp[3]) {
   double vsq = 0.;
 #pragma unroll
   for (int i = 0; i < 3; i++) vsq += vp[i] * vp[i];
-  return sqrt(1. + vsq);
+  return sqrt_p(1. + vsq);
 }
 
 enum { SUCCESS = 0, FAILURE = 1, MODIFIED = 2 };
@@ -197,7 +208,7 @@ __device__ __forceinline__ double lorentz_g(const double vp[3], const G3 &g) {
   for (int ii = 0; ii < 3; ii++)
 #pragma unroll
     for (int jj = 0; jj < 3; jj++) vsq += g.cov[ii][jj] * vp[ii] * vp[jj];
-  return sqrt(1. + vsq);
+  return sqrt_p(1. + vsq);
 }
 
 #ifdef PHX_EXACT
@@ -206,13 +217,23 @@ constexpr bool kExactBuild = true;
 constexpr bool kExactBuild = false;
 #endif
 
+// What con2prim, prim2con and the source update need of the tilde-pressure
+// tensor: v_j pi^{ij} and v_i v_j pi^{ij}.  On Minkowski
+// pi^{ij} = athin (f^i f^j - (W^2 v^i v^j + delta^{ij}) / 3) contracts in closed
+// form, so the production build's zone kernels carry these four numbers instead
+// of the tensor.
+struct PiC {
+  V3 cv;
+  double vv;
+};
+
 // ClosureEdd / ClosureM1 (M1).  MINK: the identity spatial metric, each
 // contraction over its non-zero terms; otherwise geo (the LocalThreeGeometry
 // of the zone or face) with the full 3x3 sums.
 template <bool M1, bool MINK = true>
 struct Closure {
   V3 con_v, cov_v;
-  double W, W2, iW;
+  double W, W2, iW, v2raw;
   bool robust;
   const G3 *geo;
   __device__ __forceinline__ Closure(const V3 &cv, bool rob, const G3 *g = nullptr) : robust(rob), geo(g) {
@@ -226,6 +247,7 @@ struct Closure {
     double v2 = 0.0;
 #pragma unroll
     for (int i = 0; i < 3; i++) v2 += con_v.d[i] * cov_v.d[i];
+    v2raw = v2;
     v2 = smin(v2, 0.9999);
     W = rsqrt_p(1 - v2);
     W2 = W * W;
@@ -266,7 +288,20 @@ struct Closure {
     }
     if constexpr (!MINK) geo->lower(con_vPi, cov_vPi);
   }
-  __device__ __forceinline__ void linear_source_update(double Estar, const V3 &Fs, const T2 &Pi, double JBB,
+  __device__ __forceinline__ void contractions(const PiC &Pi, V3 &cov_vPi, double &vvPi) const {
+    cov_vPi = Pi.cv;
+    vvPi = Pi.vv;
+  }
+  // athin (f (f.v) - v (W^2 v^2 + 1) / 3) and its product with v (Minkowski)
+  __device__ __forceinline__ void pic_fill(const V3 &f, double athin, PiC &Pi) const {
+    const double w3 = D3(fma(W2, v2raw, 1.0));
+    const double fv = ccov(con_v, f), a = athin * fv, c = athin * w3;
+#pragma unroll
+    for (int i = 0; i < 3; i++) Pi.cv.d[i] = fma(a, f.d[i], -c * con_v.d[i]);
+    Pi.vv = fma(a, fv, -c * v2raw);
+  }
+  template <class PIT>
+  __device__ __forceinline__ void linear_source_update(double Estar, const V3 &Fs, const PIT &Pi, double JBB,
                                                        double tauJ, double tauH, double &dE, V3 &dF) const {
     double vvPi;
     V3 cvPi;
@@ -296,7 +331,8 @@ struct Closure {
 #endif
     }
   }
-  __device__ __forceinline__ void prim2con(double J, const V3 &H, const T2 &Pi, double &E, V3 &F) const {
+  template <class PIT>
+  __device__ __forceinline__ void prim2con(double J, const V3 &H, const PIT &Pi, double &E, V3 &F) const {
     double vvPi;
     V3 cvPi;
     contractions(Pi, cvPi, vvPi);
@@ -338,7 +374,8 @@ struct Closure {
         P.d[i][j] = 4.0 / 3.0 * W2 * con_v.d[i] * con_v.d[j] * J + W * (con_v.d[i] * conH.d[j] + con_v.d[j] * conH.d[i]) +
                     J * Pi.d[i][j] + J / 3.0 * gcon(i, j);
   }
-  __device__ __forceinline__ int con2prim(double E, const V3 &F, const T2 &Pi, double &J, V3 &H) const {
+  template <class PIT>
+  __device__ __forceinline__ int con2prim(double E, const V3 &F, const PIT &Pi, double &J, V3 &H) const {
     double vvPi;
     V3 cvPi;
     contractions(Pi, cvPi, vvPi);
@@ -355,8 +392,8 @@ struct Closure {
 #pragma unroll
     for (int i = 0; i < 3; i++) H.d[i] = DW(F.d[i] - J * cvPi.d[i] - cov_v.d[i] * a);
     const double vh = ccov(con_v, H);
-    const double xi = div_p(sqrt(ccv(H, H) - vh * vh), J);
-    if (isnan(xi) || isnan(J)) return FAILURE;
+    const double xi = div_p(sqrt_p(ccv(H, H) - vh * vh), J);
+    if (is_nan(xi) || is_nan(J)) return FAILURE;
     if (J < 0. || xi >= 1.0) {
       if (robust) {
         if (J < 0.) J = smin(J, 10. * kSMALL);
@@ -418,7 +455,7 @@ struct Closure {
       for (int i = 0; i < 3; i++) Hm += H.d[i] * conH.d[i];
 #pragma unroll
       for (int i = 0; i < 3; i++) vH += H.d[i] * con_v.d[i];
-      Hm = sqrt(Hm - vH * vH);
+      Hm = sqrt_p(Hm - vH * vH);
       double f[3];
 #ifdef PHX_EXACT
 #pragma unroll
@@ -430,6 +467,33 @@ struct Closure {
 #endif
       const double xi = smax(smin(1.0, ratio_p(Hm, J)), 0.0);
       tilpi_fill(f, 0.5 * (3 * closure_fn(xi) - 1), Pi);
+    }
+  }
+  // athin of the closure at xi: (3 closure_fn - 1) / 2 = xi^2 (2 xi - 1)
+  __device__ __forceinline__ static double athin_of(double xi) { return xi * xi * fma(2.0, xi, -1.0); }
+  // 1 / sqrt(m2) of the rest-frame flux's squared magnitude and xi = H / J
+  // bounded to [0, 1]; a vanishing flux has no direction: both 0 (the
+  // reference's f = H / (H + SMALL)), NaN otherwise
+  __device__ __forceinline__ static void flux_xi(double m2, double J, double &im, double &xi) {
+    const int e = __double2hiint(m2) >> 20;
+    if (e >= 16 && e <= 2030) {
+      im = rsqrt_nr(m2);
+      xi = smax(smin(1.0, ratio_p(m2 * im, J)), 0.0);
+    } else {
+      im = xi = e >= 0 && e < 16 ? 0.0 : __longlong_as_double(0x7ff8000000000000ll);
+    }
+  }
+  __device__ __forceinline__ void tilpi_from_prim(double J, const V3 &H, PiC &Pi) const {
+    if constexpr (!M1) {
+      Pi.cv.d[0] = Pi.cv.d[1] = Pi.cv.d[2] = Pi.vv = 0.0;
+    } else {
+      const double vH = ccov(con_v, H);
+      double im, xi;
+      flux_xi(ccov(H, H) - vH * vH, J, im, xi);
+      V3 f;
+#pragma unroll
+      for (int i = 0; i < 3; i++) f.d[i] = H.d[i] * im;
+      pic_fill(f, athin_of(xi), Pi);
     }
   }
   __device__ __forceinline__ void angles_pressure(double xi, double phi, const V3 &g, const V3 &dd, T2 &Pi,
@@ -452,7 +516,7 @@ struct Closure {
     double Fmag = 0.0, vl = 0.0, vv = 0.0;
 #pragma unroll
     for (int i = 0; i < 3; i++) Fmag += F.d[i] * conF.d[i];
-    Fmag = sqrt(Fmag);
+    Fmag = sqrt_p(Fmag);
 #pragma unroll
     for (int i = 0; i < 3; i++) vl += F.d[i] * con_v.d[i];
 #ifndef PHX_EXACT
@@ -462,7 +526,7 @@ struct Closure {
 #pragma unroll
     for (int i = 0; i < 3; i++) vv += cov_v.d[i] * con_v.d[i];
     const double lam = ratio_p(1.0, W * (1 - vl));
-    const double aa = sqrt(vv * (1 + 10 * DBL_EPSILON) - vl * vl);
+    const double aa = sqrt_p(vv * (1 + 10 * DBL_EPSILON) - vl * vl);
 #ifndef PHX_EXACT
     const double iaa = rcp_p(aa + kSMALL);
 #endif
@@ -498,8 +562,8 @@ struct Closure {
     }
 #pragma unroll
     for (int i = 0; i < 3; i++) vH += con_v.d[i] * H.d[i];
-    Hm = sqrt(Hm - vH * vH);
-    return xi - ratio(Hm, J);
+    Hm = sqrt_p(Hm - vH * vH);
+    return xi - ratio_p(Hm, J);
   }
   // SolveClosure with phi held at pi (the reference's update rule keeps it
   // there); the phi-perturbed residuals only feed the discarded 2x2 solve.
@@ -629,6 +693,138 @@ struct Closure {
     xi_io = xi;
     phi_out = phi;
   }
+#ifndef PHX_EXACT
+  // SolveClosure and the tilde-pressure contractions on Minkowski (production
+  // build), phi held at pi as in solve_closure.  With the rest-frame flux
+  // direction f fixed, every quantity is a rational function of athin(xi).  The
+  // Newton iteration first runs in FP32 (one to two cycles an instruction
+  // against 64-76), then on the FP64 residual with the FP32 derivative until
+  // the residual meets the reference's tolerance.  Zones that leave the
+  // physical range on the way (J <= 0, flux factor >= 1, NaN) or do not
+  // converge at once take solve_closure from the stored xi.  f is the
+  // reference's -cos(pi) g + sin(pi) d with sin(pi) = 1.2e-16 dropped.  About 80
+  // FP64 instructions for two residuals (170 to 240 for the 2.8 to 4 FP64
+  // Newton steps of solve_closure); 96^3 stage, first pass on a new state, 8.2
+  // -> 3.9 ms with the closed-form face states and contractions.
+  __device__ __forceinline__ bool closure_fast(double E0, const V3 &F0, double &xi, PiC &Pi) const {
+    const double tol = 1.e6 * DBL_EPSILON;
+    const double iE = ratio_p(1.0, E0);
+    V3 F, f;
+#pragma unroll
+    for (int i = 0; i < 3; i++) F.d[i] = F0.d[i] * iE + (gt(0.0, F0.d[i]) ? -1.e3 * DBL_MIN : 1.e3 * DBL_MIN);
+    // basis(): g = lam F / |F| - W v, lam = 1 / (W (1 - v.F / |F|))
+    const double F2 = ccov(F, F), vF = ccov(con_v, F);
+    const int eF = __double2hiint(F2) >> 20;
+    if (!(eF >= 16 && eF <= 2030)) return false;
+    const double iF = rsqrt_nr(F2);
+    const double q = iF * rcp_p(W * fma(-vF, iF, 1.0));
+#pragma unroll
+    for (int i = 0; i < 3; i++) f.d[i] = fma(q, F.d[i], -W * con_v.d[i]);
+    pic_fill(f, 1.0, Pi);  // C0, V0: the contractions at athin = 1
+    const V3 C0 = Pi.cv;
+    const double V0 = Pi.vv;
+    const double L0 = D3(2.0 * W2 + 1.0), c1 = (2.0 * W2 - 3.0) * W2;
+    const double NJ = (2 * W2 - 1) - 2 * W2 * vF;
+    const double K0 = D3(4 * W2) - D3(4 * W2 + 1) * vF, Kv = W2 * vF - 1.0;
+    const float fV0 = d2f_bits(V0), fL0 = d2f_bits(L0), fc1 = d2f_bits(c1), fNJ = d2f_bits(NJ), fK0 = d2f_bits(K0),
+                fKv = d2f_bits(Kv), fW2 = d2f_bits(W2), fiW = d2f_bits(iW);
+    float fF[3], fC[3], fv[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      fF[i] = d2f_bits(F.d[i]);
+      fC[i] = d2f_bits(C0.d[i]);
+      fv[i] = d2f_bits(con_v.d[i]);
+    }
+    float x = d2f_bits(xi), d = 1.0f;
+    if (!(x >= 0.0f && x <= 1.0f)) return false;
+#pragma unroll 1
+    for (int it = 0; it < 10; it++) {
+      const float at = x * x * fmaf(2.0f, x, -1.0f), dat = x * fmaf(6.0f, x, -2.0f);
+      const float V = at * fV0, dV = dat * fV0;
+      const float ilam = rcp_f32(fmaf(fc1, V, fL0));
+      const float K = fmaf(V, fKv, fK0);
+      const float J = fNJ * ilam, A = fW2 * ilam * K, Ja = J * at;
+      const float dil = -fc1 * dV * ilam * ilam;
+      const float dJ = fNJ * dil, dA = fW2 * fmaf(dil, K, ilam * fKv * dV), dJa = fmaf(dJ, at, J * dat);
+      float hh = 0.0f, vh = 0.0f, hd = 0.0f, vd = 0.0f;
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const float h = (fF[i] - Ja * fC[i] - fv[i] * A) * fiW, dh = -(fmaf(dJa, fC[i], fv[i] * dA)) * fiW;
+        hh = fmaf(h, h, hh);
+        vh = fmaf(fv[i], h, vh);
+        hd = fmaf(h, dh, hd);
+        vd = fmaf(fv[i], dh, vd);
+      }
+      const float s2 = fmaxf(hh - vh * vh, 1e-30f), is = rsqrt_f32(s2), s0 = s2 * is, iJ = rcp_f32(J);
+      d = 1.0f - ((hd - vh * vd) * is - s0 * dJ * iJ) * iJ;
+      const float xc = s0 * iJ;
+      if (!(J > 0.0f && xc < 1.0f && d > 0.05f && d < 20.0f)) return false;
+      // a step out of [0, 1] meets the reference's clamps: its own solve decides
+      const float n = x - (x - xc) * rcp_f32(d);
+      if (!(n >= 0.0f && n <= 1.0f)) return false;
+      const float ch = fabsf(n - x);
+      x = n;
+      if (ch <= 3e-7f) break;
+    }
+    const double id = f2d_bits(rcp_f32(d));
+    double y = f2d_bits(x), at;
+#pragma unroll 1
+    for (int it = 0;; it++) {
+      at = athin_of(y);
+      const double ilam = ratio_p(1.0, fma(c1 * V0, at, L0));
+      const double A = W2 * ilam * fma(at * V0, Kv, K0);
+      const double J = NJ * ilam;
+      const double Ja = J * at;
+      V3 H;
+#pragma unroll
+      for (int i = 0; i < 3; i++) H.d[i] = (fma(-Ja, C0.d[i], F.d[i]) - con_v.d[i] * A) * iW;
+      const double vh = ccov(con_v, H);
+      const double xc = div_p(sqrt_p(ccov(H, H) - vh * vh), J);
+      if (!gt(J, 0.0) || !gt(1.0, xc) || it == 4) return false;
+      const double r = y - xc;
+      y -= r * id;
+      if (!gt(y, -tol) || gt(y, 1.0)) return false;
+      if (!gt(fabs(r), tol)) break;
+    }
+    y = clamp0(y);
+    at = athin_of(y);
+#pragma unroll
+    for (int i = 0; i < 3; i++) Pi.cv.d[i] = C0.d[i] * at;
+    Pi.vv = V0 * at;
+    xi = y;
+    return true;
+  }
+  __device__ __forceinline__ void tilpi_from_con(double E0, const V3 &F0, double &xi, double &phi, PiC &Pi) const {
+    if constexpr (!M1) {
+      Pi.cv.d[0] = Pi.cv.d[1] = Pi.cv.d[2] = Pi.vv = 0.0;
+      xi = 0.0;
+      phi = PI;
+    } else if (is_nan(E0) || is_nan(F0.d[0]) || is_nan(F0.d[1]) || is_nan(F0.d[2]) || is_nan(xi)) {
+      // solve_closure's outcome
+      xi = phi = Pi.vv = Pi.cv.d[0] = Pi.cv.d[1] = Pi.cv.d[2] = __longlong_as_double(0x7ff8000000000000ll);
+    } else if (closure_fast(E0, F0, xi, Pi)) {
+      phi = PI;
+    } else {
+      const ClosureTry t = closure_slow(*this, E0, F0, xi);
+      xi = t.xi;
+      phi = t.phi;
+      Pi = t.Pi;
+    }
+  }
+  // The reference's solve, kept out of the callers' instruction stream.
+  struct ClosureTry {
+    double xi, phi;
+    PiC Pi;
+  };
+  static __device__ __noinline__ ClosureTry closure_slow(Closure c, double E0, V3 F0, double xi0) {
+    ClosureTry t;
+    t.xi = xi0;
+    T2 Pi;
+    c.tilpi_from_con(E0, F0, t.xi, t.phi, Pi);
+    c.contractions(Pi, t.Pi.cv, t.Pi.vv);
+    return t;
+  }
+#endif
   // GetConTilPiFromCon
   __device__ __forceinline__ void tilpi_from_con(double E, const V3 &F, double &xi, double &phi, T2 &Pi) const {
     if constexpr (!M1) {
@@ -692,9 +888,15 @@ __device__ __forceinline__ V3 fluid_v(const BView &b, long long id, const G3 *g 
     W = lorentz_g(vp, *g);
   if (Wout) *Wout = W;
   V3 v;
+#ifdef PHX_EXACT
   v.d[0] = vp[0] / W;
   v.d[1] = vp[1] / W;
   v.d[2] = vp[2] / W;
+#else
+  const double iW = rcp_p(W);
+#pragma unroll
+  for (int a = 0; a < 3; a++) v.d[a] = vp[a] * iW;
+#endif
   return v;
 }
 __device__ __forceinline__ void zone_of(const Range3 &r, long long t, int &k, int &j, int &i) {
@@ -706,6 +908,10 @@ __device__ __forceinline__ void zone_of(const Range3 &r, long long t, int &k, in
 __host__ __device__ inline long long range_count(const Range3 &r) {
   return (long long)(r.ie - r.is + 1) * (r.je - r.js + 1) * (r.ke - r.ks + 1);
 }
+
+// The zone kernels' representation of the tilde-pressure tensor.
+template <bool M1, bool MINK>
+using ZonePi = std::conditional_t<M1 && MINK && !kExactBuild, PiC, T2>;
 
 // ---------------------------------------------------- MomentPrim2Con
 template <bool M1, bool MINK>
@@ -721,7 +927,7 @@ __global__ void __launch_bounds__(128) k_p2c(RPar p, BView b, RView r, Range3 rg
   V3 H;
 #pragma unroll
   for (int a = 0; a < 3; a++) H.d[a] = r.prim[(PHX_RH + a) * vs + id] * J;
-  T2 Pi;
+  ZonePi<M1, MINK> Pi;
   c.tilpi_from_prim(J, H, Pi);
   double E;
   V3 F;
@@ -752,7 +958,7 @@ __global__ void __launch_bounds__(128) k_c2p(RPar p, BView b, RView r, Range3 rg
     xi = r.prim[PHX_RXI * vs + id];
     phi = 1.0001 * r.prim[PHX_RPHI * vs + id];
   }
-  T2 Pi;
+  ZonePi<M1, MINK> Pi;
   c.tilpi_from_con(E, F, xi, phi, Pi);
   if constexpr (M1) {
     r.prim[PHX_RXI * vs + id] = xi;
@@ -814,6 +1020,35 @@ __device__ __forceinline__ void face_state(const Closure<M1, MINK> &c, double J,
     Fd = conF.d[d] * c.geo->alpha;
   }
 }
+
+#ifndef PHX_EXACT
+// The M1 face state on Minkowski with the tilde-pressure tensor contracted in
+// closed form (production build): with Ja = athin J and q = Ja / H^2,
+// J pi^{ij} = q H^i H^j - Ja (W^2 v^i v^j + delta^{ij}) / 3.  About 45 FP64
+// instructions (130 through the tensor): 96^3, three directions, 3.3 -> 1.95 ms.
+template <int d>
+__device__ __forceinline__ void face_state(const Closure<true, true> &c, double J, const V3 &H, double &E, V3 &F,
+                                           double &Fd, double P[3], int) {
+  const V3 &v = c.con_v;
+  const double vH = ccov(v, H);
+  double im, xi;
+  c.flux_xi(ccov(H, H) - vH * vH, J, im, xi);
+  const double Ja = J * c.athin_of(xi);
+  const double q = Ja * (im * im), qvH = q * vH;
+  const double w3 = Ja * D3(fma(c.W2, c.v2raw, 1.0));
+  const double a43 = D3(4 * c.W2) * J;
+  const double vvPi = fma(qvH, vH, -w3 * c.v2raw);
+  E = fma(c.W2, vvPi, fma(2.0 * c.W, vH, a43 - D3(J)));
+  const double av = fma(c.W, vH, a43 - w3), ah = c.W + qvH;
+#pragma unroll
+  for (int j = 0; j < 3; j++) F.d[j] = fma(av, v.d[j], ah * H.d[j]);
+  const double pv = fma(v.d[d], fma(-D3(c.W2), Ja, a43), c.W * H.d[d]), ph = fma(q, H.d[d], c.W * v.d[d]);
+#pragma unroll
+  for (int j = 0; j < 3; j++) P[j] = fma(pv, v.d[j], ph * H.d[j]);
+  P[d] += D3(J - Ja);
+  Fd = F.d[d];
+}
+#endif
 
 template <bool M1, int RECON, int d, bool MINK>
 __global__ void __launch_bounds__(128) k_fluxes(RPar p, BView b, RView r, Range3 rg) {
@@ -920,8 +1155,8 @@ __global__ void __launch_bounds__(128) k_fluxes(RPar p, BView b, RView r, Range3
     const double vhl = ccov(vl, Hl), vhr = ccov(vr, Hr);
     const double hhl = MINK ? ccov(Hl, Hl) : G.g.contract_cov(Hl, Hl);
     const double hhr = MINK ? ccov(Hr, Hr) : G.g.contract_cov(Hr, Hr);
-    const double xil = div_p(sqrt(hhl - vhl * vhl), Jl);
-    const double xir = div_p(sqrt(hhr - vhr * vhr), Jr);
+    const double xil = div_p(sqrt_p(hhl - vhl * vhl), Jl);
+    const double xir = div_p(sqrt_p(hhr - vhr * vhr), Jr);
     if (xil > p.xi_ceiling) {
 #pragma unroll
       for (int a = 0; a < 3; a++) Hl.d[a] *= p.xi_ceiling / xil;
@@ -932,8 +1167,8 @@ __global__ void __launch_bounds__(128) k_fluxes(RPar p, BView b, RView r, Range3
     }
   }
   const double *kH = r.prim + PHX_RKAPPAH * vs;
-  const double kappaH = sqrt(kH[id] * kH[idm]);
-  const double aw = tanh_r(ratio(1.0, fabs(kappaH * dx)));
+  const double kappaH = sqrt_p(kH[id] * kH[idm]);
+  const double aw = tanh_r(ratio_p(1.0, fabs(kappaH * dx)));
   const double kappaH_min = 1.e-20;
   V3 Has;
 #ifdef PHX_EXACT
@@ -947,10 +1182,20 @@ __global__ void __launch_bounds__(128) k_fluxes(RPar p, BView b, RView r, Range3
   const Closure<M1, MINK> cl(vl, true, G.geo()), cr(vr, true, G.geo());
   double El, Er, Fdl, Fdr, Fdl_a, Fdr_a, Pl[3], Pr[3], Pl_a[3], Pr_a[3], Ed;
   V3 Fl, Fr, Fd_scr;
-  face_state<M1, d, MINK>(cl, Jl, Has, Ed, Fd_scr, Fdl_a, Pl_a);
-  face_state<M1, d, MINK>(cr, Jr, Has, Ed, Fd_scr, Fdr_a, Pr_a);
-  face_state<M1, d, MINK>(cl, Jl, Hl, El, Fl, Fdl, Pl);
-  face_state<M1, d, MINK>(cr, Jr, Hr, Er, Fr, Fdr, Pr);
+#ifndef PHX_EXACT
+  if constexpr (M1 && MINK) {
+    face_state<d>(cl, Jl, Has, Ed, Fd_scr, Fdl_a, Pl_a, 0);
+    face_state<d>(cr, Jr, Has, Ed, Fd_scr, Fdr_a, Pr_a, 0);
+    face_state<d>(cl, Jl, Hl, El, Fl, Fdl, Pl, 0);
+    face_state<d>(cr, Jr, Hr, Er, Fr, Fdr, Pr, 0);
+  } else
+#endif
+  {
+    face_state<M1, d, MINK>(cl, Jl, Has, Ed, Fd_scr, Fdl_a, Pl_a);
+    face_state<M1, d, MINK>(cr, Jr, Has, Ed, Fd_scr, Fdr_a, Pr_a);
+    face_state<M1, d, MINK>(cl, Jl, Hl, El, Fl, Fdl, Pl);
+    face_state<M1, d, MINK>(cr, Jr, Hr, Er, Fr, Fdr, Pr);
+  }
   Fdl = aw * Fdl + (1 - aw) * Fdl_a;
   Fdr = aw * Fdr + (1 - aw) * Fdr_a;
 #pragma unroll
@@ -1126,6 +1371,30 @@ struct TRes {
   }
 #endif
 };
+// a / b as the IEEE division rounds it: the production build corrects
+// a rcp(b) by its exact remainder (three FP64 instructions), which gives the
+// correctly rounded quotient.  The iteration below fails a zone that needs
+// more than its iteration cap -- near equilibrium it takes 70 to 100 of them,
+// its end value only moving through the halvings -- so its steps stay the
+// reference's.
+__device__ __forceinline__ double div_ieee(double a, double b) {
+#ifndef PHX_EXACT
+  const int eb = dexp(b), ea = dexp(a);
+  if (eb >= 64 && eb <= 1982 && ea >= 128 && ea <= 1918) {
+    const double r = rcp_nr(b), q = a * r;
+    const int eq = dexp(q);
+    if (eq >= 64 && eq <= 1982) return fma(fma(-b, q, a), r, q);
+  }
+#endif
+  return a / b;
+}
+__device__ __forceinline__ bool same(double a, double b) {
+#ifdef PHX_EXACT
+  return a == b;
+#else
+  return !gt(a, b) && !gt(b, a) && !is_nan(a) && !is_nan(b);
+#endif
+}
 // RootFind::regula_falsi with a status; the iteration count persists across
 // calls (the reference reuses one RootFind for its re-bracketing tries).
 __device__ __forceinline__ double regula_falsi(const TRes &f, double a, double b, double tol, double guess,
@@ -1153,25 +1422,25 @@ __device__ __forceinline__ double regula_falsi(const TRes &f, double a, double b
   ya *= sign;
   yb *= sign;
   int b1 = 0, b2 = 0;
-  while (b - a > 2.0 * tol && count < max_iter) {
-    const double c = (a * yb - b * ya) / (yb - ya);
-    if (c == a) {
+  while (gt(b - a, 2.0 * tol) && count < max_iter) {
+    const double c = div_ieee(a * yb - b * ya, yb - ya);
+    if (same(c, a)) {
       b = a;
       count++;
       continue;
-    } else if (c == b) {
+    } else if (same(c, b)) {
       a = b;
       count++;
       continue;
     }
     const double yc = sign * f(c);
-    if (yc > 0.0) {
+    if (gt(yc, 0.0)) {
       b = c;
       yb = yc;
       b1++;
       ya *= (b1 > 1 ? 0.5 : 1.0);
       b2 = 0;
-    } else if (yc < 0.0) {
+    } else if (gt(0.0, yc)) {
       a = c;
       ya = yc;
       b2++;
@@ -1553,7 +1822,7 @@ __global__ void __launch_bounds__(128) k_source(RPar p, Par fp, BView b, RView r
   V3 dF;
   dF.d[0] = dF.d[1] = dF.d[2] = 0.0;
   bool success = false;
-  T2 Pi;
+  ZonePi<M1, MINK> Pi;
   bool oned = !FOURD;
   if constexpr (FOURD) {
     // fourd, falling back to oned when it fails and src_use_oned_backup is
@@ -1564,7 +1833,7 @@ __global__ void __launch_bounds__(128) k_source(RPar p, Par fp, BView b, RView r
   }
   if (oned) {
     const double J0 = r.prim[PHX_RJ * vs + id];
-    const double dtau = alpha * dt / W;
+    const double dtau = div_p(alpha * dt, W);
     TRes res{&p, rho, ug, J0, dtau, amax};
     res.prepare();
     int count = 0;
