@@ -109,7 +109,9 @@ void launch_fluxct(const BView &b, cudaStream_t s) {
 __device__ __forceinline__ void update_at(const BView &b, const double *base, double *out, double beta, double bdt,
                                           int ncons, long long t) {
   const double dx1 = b.dx[0], dx2 = b.dx[1], dx3 = b.dx[2];
+#ifdef PHX_EXACT
   const double A1 = dx2 * dx3, A2 = dx1 * dx3, A3 = dx1 * dx2, V = dx1 * dx2 * dx3;
+#endif
   const int ni = b.nx1, nj = b.ndim >= 2 ? b.nx2 : 1;
   const int i = b.ng + (int)(t % ni);
   const int j = (b.ndim >= 2 ? b.ng : 0) + (int)((t / ni) % nj);
@@ -117,17 +119,36 @@ __device__ __forceinline__ void update_at(const BView &b, const double *base, do
   const long long id = b.idx(k, j, i);
   const long long dk = (long long)b.n1t * b.n2t, dj = b.n1t;
 #ifndef PHX_EXACT
-  const double iV = rcp_p(V);  // one reciprocal for the ncons divisions by the volume
-#endif
+  // production build: A_d / V = 1 / dx_d, and beta = 1 (a first stage) leaves
+  // u0 = cons as it stands unless base is not finite (0 * base is then NaN): 7
+  // to 10 FP64 instructions per variable instead of 14, and a first stage does
+  // not write cons
+  const double c1 = rcp_p(dx1), c2 = rcp_p(dx2), c3 = rcp_p(dx3);
+  const bool first = __double_as_longlong(beta) == 0x3ff0000000000000ll;
+#pragma unroll 4
+  for (int m = 0; m < ncons; m++) {
+    double r = c1 * (FX(b, 0, m, id) - FX(b, 0, m, id + 1));
+    if (b.ndim >= 2) r = fma(c2, FX(b, 1, m, id) - FX(b, 1, m, id + dj), r);
+    if (b.ndim == 3) r = fma(c3, FX(b, 2, m, id) - FX(b, 2, m, id + dk), r);
+    if (m >= 1 && m <= 4 && b.src != nullptr) r = r + b.src[(m - 1) * b.vs + id];
+    const long long vid = m * b.vs + id;
+    if (b.dudt != nullptr) b.dudt[vid] = r;
+    if (out != nullptr) {
+      const double v0 = base[vid];
+      double u0 = b.cons[vid];
+      if (!first || (__double2hiint(v0) & 0x7ff00000) == 0x7ff00000) {
+        u0 = beta * u0 + (1 - beta) * v0;
+        b.cons[vid] = u0;
+      }
+      out[vid] = fma(bdt, r, u0);
+    }
+  }
+#else
   for (int m = 0; m < ncons; m++) {
     double du = (A1 * FX(b, 0, m, id + 1) - A1 * FX(b, 0, m, id));
     if (b.ndim >= 2) du += A2 * FX(b, 1, m, id + dj) - A2 * FX(b, 1, m, id);
     if (b.ndim == 3) du += A3 * FX(b, 2, m, id + dk) - A3 * FX(b, 2, m, id);
-#ifdef PHX_EXACT
     double r = -du / V;
-#else
-    double r = -du * iV;
-#endif
     if (m >= 1 && m <= 4 && b.src != nullptr) r = r + b.src[(m - 1) * b.vs + id];
     const long long vid = m * b.vs + id;
     if (b.dudt != nullptr) b.dudt[vid] = r;
@@ -138,6 +159,7 @@ __device__ __forceinline__ void update_at(const BView &b, const double *base, do
       out[vid] = u0 + bdt * r;
     }
   }
+#endif
 }
 
 __global__ void __launch_bounds__(256) k_update(BView b, const double *base, double *out, double beta,
@@ -269,14 +291,6 @@ __device__ __forceinline__ void sources_at(const Par &p, const BView &b, long lo
         Bdotv += bf[ii] * (vp[jj] / W) * g.gcov[ii + 1][jj + 1];
         Bsq += bf[ii] * bf[jj] * g.gcov[ii + 1][jj + 1];
       }
-#else
-    double vlo[3], blo[3];  // the lowered vectors serve the three contractions
-    lower_sp(g, vp, vlo);
-    lower_sp(g, bf, blo);
-    const double W = sqrt(1. + dot3(vp, vlo));
-    const double Bdotv = div_p(dot3(bf, vlo), W);
-    const double Bsq = dot3(bf, blo);
-#endif
     const double iW = ratio_p(1., W);
     const double alpha = g.alpha;
     double u[4], bb[4];
@@ -334,6 +348,76 @@ __device__ __forceinline__ void sources_at(const Par &p, const BView &b, long lo
     for (int d = 1; d < 4; d++) da[d] = __ldg(b.gderiv + (PHX_GD_DALPHA + d - 1) * pitch + off);
     for (int m = 0; m < 4; m++) Ta += T[m][0] * da[m];
     b.src[3 * vs + id] = gdet * alpha * (Ta - TGam);
+#else
+    // production build, with T symmetric: T^{mn} (d_m g_{nl} - Gamma_{l,nm}) =
+    // T^{mn} d_l g_{mn} / 2 =: S_l, and T^{mn} Gamma_{r,mn} = T^{mn} d_n g_{mr} - S_r
+    // (S_0 = 0): about 200 FP64 instructions instead of 450.  With the update's,
+    // 96^3 torus stage 10.6 -> 10.1 ms, a 128-zone 1D stage 100 -> 90 us (the
+    // chain of one zone's instructions)
+    double vlo[3], blo[3];
+    lower_sp(g, vp, vlo);
+    lower_sp(g, bf, blo);
+    const double Wsq = 1. + dot3(vp, vlo);
+    const double iW = rsqrt_p(Wsq), W = Wsq * iW;
+    const double Bdotv = dot3(bf, vlo) * iW;
+    const double alpha = g.alpha, ialpha = ratio_p(1., alpha);
+    double u[4], bb[4];
+    u[0] = W * fabs(ialpha);
+    bb[0] = u[0] * Bdotv;
+    const double ab0 = alpha * bb[0];
+#pragma unroll
+    for (int l = 1; l < 4; ++l) {
+      u[l] = fma(-u[0], g.beta[l - 1], vp[l - 1]);
+      bb[l] = iW * fma(ab0, u[l], bf[l - 1]);
+    }
+    const double bsq = fma(dot3(bf, blo), iW * iW, Bdotv * Bdotv);
+    const double ia2 = ialpha * ialpha;
+    double gc0[4] = {-ia2, g.beta[0] * ia2, g.beta[1] * ia2, g.beta[2] * ia2};  // g^{0 mu}
+    const double A = rho + uu + Pr + bsq, Bt = fma(0.5, bsq, Pr);
+    double T[4][4], T0[4];  // T0: A u^mu
+#pragma unroll
+    for (int mu = 0; mu < 4; mu++) T0[mu] = A * u[mu];
+#pragma unroll
+    for (int mu = 0; mu < 4; mu++)
+#pragma unroll
+      for (int nu = mu; nu < 4; nu++) {
+        const double gi = mu == 0 ? gc0[nu] : fma(-g.beta[mu - 1], gc0[nu], g.gamcon[mu - 1][nu - 1]);
+        T[mu][nu] = T[nu][mu] = fma(T0[mu], u[nu], fma(Bt, gi, -bb[mu] * bb[nu]));
+      }
+    const double gdet = alpha * g.detgam;
+    const long long pitch = (long long)b.n2t * b.n1t, off = (long long)j * b.n1t + i;
+    const double *dgt = b.gderiv + PHX_GD_DG * pitch + off;
+    // dg(mu, nu, s) = d_s g_{mu nu}, s = 1..3
+    double S[4] = {0.0, 0.0, 0.0, 0.0}, TGam = 0.0;
+    double Z[4][3];  // Z[m][s-1] = g^{0 r} d_s g_{m r}
+#pragma unroll
+    for (int s = 1; s < 4; s++) {
+      double sum = 0.0;
+#pragma unroll
+      for (int m = 0; m < 4; m++) Z[m][s - 1] = 0.0;
+#pragma unroll
+      for (int mu = 0; mu < 4; mu++)
+#pragma unroll
+        for (int nu = mu; nu < 4; nu++) {
+          const double d = __ldg(dgt + (3 * flat2(mu, nu) + s - 1) * pitch);
+          sum = mu == nu ? fma(0.5 * T[mu][mu], d, sum) : fma(T[mu][nu], d, sum);
+          Z[mu][s - 1] = fma(gc0[nu], d, Z[mu][s - 1]);
+          if (mu != nu) Z[nu][s - 1] = fma(gc0[mu], d, Z[nu][s - 1]);
+        }
+      S[s] = sum;
+      b.src[(s - 1) * vs + id] = gdet * sum;
+    }
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+#pragma unroll
+      for (int s = 1; s < 4; s++) TGam = fma(T[m][s], Z[m][s - 1], TGam);
+#pragma unroll
+    for (int s = 1; s < 4; s++) TGam = fma(-gc0[s], S[s], TGam);
+    double Ta = 0.0;
+#pragma unroll
+    for (int d = 1; d < 4; d++) Ta = fma(T[d][0], __ldg(b.gderiv + (PHX_GD_DALPHA + d - 1) * pitch + off), Ta);
+    b.src[3 * vs + id] = gdet * alpha * (Ta - TGam);
+#endif
   }
 }
 
