@@ -161,6 +161,7 @@ phx_status make_view(const phx_block *b, phx::BView &v) {
   v.src = b->src;
   v.emf = b->emf;
   v.dudt = b->dudt;
+  v.flr = nullptr;
   v.fmks = 0;
   v.gcent = v.gface1 = v.gface2 = v.gderiv = nullptr;
   if (b->geom && b->geom->kind == PHX_GEOM_FMKS) {

@@ -488,8 +488,15 @@ cudaError_t batch_stage(BatchCache *cache, const Par &par, const phx_block *bloc
     P.ndim = views[0].ndim;
     std::vector<BView> vin(views, views + n), vout(views, views + n);
     for (int i = 0; i < n; i++) vout[i].cons = out[i];
+    // floor tables, where the floors vary along X1 alone (their bounds and the
+    // blocks' grids are part of the plan's identity)
+    const bool floor_tab = par.floor_type == PHX_FLOOR_EXPX1_RHO_SIE || par.floor_type == PHX_FLOOR_EXPX1_RHO_U ||
+                           par.floor_type == PHX_FLOOR_X1_RHO_SIE;
+    size_t nfloor = 0;
+    if (floor_tab)
+      for (const BView &v : vin) nfloor += 2 * (size_t)v.n1t + 1;
     const size_t bytes = 2 * sizeof(BView) * n + 2 * sizeof(double *) * n + 2 * sizeof(double) +
-                         sizeof(CUtensorMap) * n + sizeof(int) * n + 256 * 10;
+                         sizeof(CUtensorMap) * n + sizeof(int) * n + sizeof(double2) * nfloor + 256 * 11;
     if ((e = cudaMalloc(&P.mem, bytes)) != cudaSuccess) return e;
     char *m = static_cast<char *>(P.mem);
     auto take = [&](size_t b) {
@@ -513,6 +520,15 @@ cudaError_t batch_stage(BatchCache *cache, const Par &par, const phx_block *bloc
       }
       cudaMemcpy(P.x1_maps, maps.data(), sizeof(CUtensorMap) * n, cudaMemcpyHostToDevice);
       cudaMemcpy(P.x1_modes, modes.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
+    }
+    if (floor_tab) {
+      double2 *t = reinterpret_cast<double2 *>(take(sizeof(double2) * nfloor));
+      for (int i = 0; i < n; i++) {
+        launch_floor_table(par, vin[i], t, 0);
+        vin[i].flr = vout[i].flr = t;
+        t += 2 * (size_t)vin[i].n1t + 1;
+      }
+      if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(0)) != cudaSuccess) return e;
     }
     cudaMemcpy(P.views_in, vin.data(), sizeof(BView) * n, cudaMemcpyHostToDevice);
     cudaMemcpy(P.views_out, vout.data(), sizeof(BView) * n, cudaMemcpyHostToDevice);

@@ -112,7 +112,7 @@ void launch_p2c_zones(const Par &p, long long n, const double *prim, const doubl
 // per-zone geometry.  The learned start runs as two kernels per chunk of
 // zones: k_mlp_bracket (setup invariants -> tensor-core network -> bracket
 // (m, lo, hi), 24 bytes per zone in a context scratch) and k_c2p<LEARNED>,
-// whose unchanged FP64 root find starts from that bracket.  Keeping the
+// whose root find starts from that bracket.  Keeping the
 // network out of the root-find kernel keeps that kernel's instruction
 // footprint small (fused, the two codes thrashed the instruction cache).
 constexpr int C2P_THREADS = 128;
@@ -133,7 +133,7 @@ struct BoxZones {
   }
   template <bool MINK>
   __device__ __forceinline__ void load(long long t, long long &id, Pt &g, double U[PHX_NCONS], double &x1, double &x2,
-                                       double &x3, double &guess) const {
+                                       double &x3, double &guess, const double2 *&flr) const {
     int k, j, i;
     id = this->id(t, k, j, i);
     if constexpr (!MINK) load_pt(b, 0, j, i, g);
@@ -143,6 +143,7 @@ struct BoxZones {
     x2 = b.Xc(1, j);
     x3 = b.Xc(2, k);
     guess = b.prim[PHX_PMU * b.vs + id];
+    flr = floor_cell(b, i);
   }
   // the stored mu of zone t alone (the learned start's cold-zone test)
   __device__ __forceinline__ double guess_of(long long t) const {
@@ -176,7 +177,7 @@ struct ListZones {
   const double *geom, *coords;
   template <bool MINK>
   __device__ __forceinline__ void load(long long t, long long &id, Pt &g, double U[PHX_NCONS], double &x1, double &x2,
-                                       double &x3, double &guess) const {
+                                       double &x3, double &guess, const double2 *&flr) const {
     id = t;
     if constexpr (!MINK) load_pt_flat(geom, n, t, g);
 #pragma unroll
@@ -185,6 +186,7 @@ struct ListZones {
     x2 = coords ? coords[n + t] : 0.0;
     x3 = coords ? coords[2 * n + t] : 0.0;
     guess = prim ? prim[PHX_PMU * n + t] : 0.0;
+    flr = nullptr;
   }
   __device__ __forceinline__ double guess_of(long long t) const { return prim ? prim[PHX_PMU * n + t] : 0.0; }
   __device__ __forceinline__ void store(long long id, const Par &p, const double pr[PHX_NPRIM],
@@ -240,7 +242,8 @@ __global__ void __launch_bounds__(C2P_THREADS) k_mlp_bracket(Par p, Z zones, lon
       long long id;
       Pt g{};
       double U[PHX_NCONS], x1, x2, x3, guess;
-      zones.template load<MINK>(t0 + q, id, g, U, x1, x2, x3, guess);
+      const double2 *flr;
+      zones.template load<MINK>(t0 + q, id, g, U, x1, x2, x3, guess, flr);
       ok = c2p_features_fp32<MINK>(p, g, U, x1, x2, x3, f) && mlp_in_box(S->w, f);
     }
     if (!__syncthreads_or(cold)) continue;  // whole chunk warm: no network
@@ -320,9 +323,11 @@ __device__ __forceinline__ bool c2p_complete(const Par &p, const Z &zones, long 
   return success;
 }
 
-// Zones whose root find is still running after the first kernel's iteration
-// cap: chunk offset and the saved RFState (it, evals, b1, b2 in 16/16/14/14
-// bits, then the sign and learned bits).
+// Zones left to the retry launch: chunk offset and, in the exact build (whose
+// first kernel stops at an iteration cap), the saved RFState (it, evals, b1, b2
+// in 16/16/14/14 bits, then the sign and learned bits).  The production
+// build's list holds the zones its fast root did not accept, which start
+// again from the reference's bracket.
 struct RetryBuf {
   int *count;
   int *idx;
@@ -372,8 +377,9 @@ __global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK)) k_c2p(Par p, Z zo
   double rcon[3], rcov[3], bu[3], Bprim[3] = {0.0, 0.0, 0.0}, bdotr = 0.0, guess = 0.0;
   if (valid) {
     double x1, x2, x3;
-    zones.template load<MINK>(t0 + q, id, g, U, x1, x2, x3, guess);
-    setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr);
+    const double2 *flr;
+    zones.template load<MINK>(t0 + q, id, g, U, x1, x2, x3, guess, flr);
+    setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr, flr);
   }
   const bool run = valid && setup_ok;
   double lb[3] = {0.0, 0.0, 0.0};
@@ -448,8 +454,9 @@ __global__ void __launch_bounds__(C2P_THREADS) k_c2p_retry(Par p, Z zones, long 
     RFState st{};
     if (valid) {
       double x1, x2, x3;
-      zones.template load<MINK>(t0 + rb.idx[k], id, g, U, x1, x2, x3, guess);
-      setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr);
+      const double2 *flr;
+      zones.template load<MINK>(t0 + rb.idx[k], id, g, U, x1, x2, x3, guess, flr);
+      setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr, flr);
 #ifdef PHX_EXACT
       st.a = rb.a[k];
       st.b = rb.b[k];
@@ -489,7 +496,9 @@ static void launch_bracket_any(const Par &p, const Z &z, long long t0, long long
 }
 
 // Zones per chunk of C2P_CHUNK; per chunk: [bracket launch], root-find
-// launch with an iteration cap, retry launch over the deferred zones.  The
+// launch, retry launch over the deferred zones.  In the exact build the
+// root-find launch has an iteration cap (the production build's fast root ends
+// by itself and takes none); the
 // caps default to a little above the mean iteration count of each start on
 // Kerr-Schild zones at tolerance 1e-10; PHX_C2P_CAP_PLAIN /
 // PHX_C2P_CAP_LEARNED in the environment override them (read once).
@@ -591,7 +600,8 @@ __global__ void __launch_bounds__(C2P_THREADS) kb_mlp_bracket(Par p, const BView
       long long id;
       Pt g{};
       double U[PHX_NCONS], x1, x2, x3, guess;
-      zones.template load<MINK>(q, id, g, U, x1, x2, x3, guess);
+      const double2 *flr;
+      zones.template load<MINK>(q, id, g, U, x1, x2, x3, guess, flr);
       ok = c2p_features_fp32<MINK>(p, g, U, x1, x2, x3, f) && mlp_in_box(S->w, f);
     }
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
@@ -657,8 +667,9 @@ __global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK)) kb_c2p(Par p, con
     double rcon[3], rcov[3], bu[3], Bprim[3] = {0.0, 0.0, 0.0}, bdotr = 0.0, guess = 0.0;
     if (valid) {
       double x1, x2, x3;
-      zones.template load<MINK>(q, id, g, U, x1, x2, x3, guess);
-      setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr);
+      const double2 *flr;
+      zones.template load<MINK>(q, id, g, U, x1, x2, x3, guess, flr);
+      setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr, flr);
     }
     double lb[3] = {0.0, 0.0, 0.0};
     if constexpr (LEARNED) {
@@ -723,8 +734,9 @@ __global__ void __launch_bounds__(C2P_THREADS) kb_ox1_inflow(Par p, const BView 
     double rcon[3], rcov[3], bu[3], Bprim[3] = {0.0, 0.0, 0.0}, bdotr = 0.0, guess = 0.0;
     if (valid) {
       double x1, x2, x3;
-      zones.template load<false>(q, id, g, U, x1, x2, x3, guess);
-      setup_ok = c2p_setup<false>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr);
+      const double2 *flr;
+      zones.template load<false>(q, id, g, U, x1, x2, x3, guess, flr);
+      setup_ok = c2p_setup<false>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr, flr);
     }
     C2POut out{0, 0, false, true, false, false};
     const double mu = c2p_root_warp<false>(p, res, valid && setup_ok, guess, out);

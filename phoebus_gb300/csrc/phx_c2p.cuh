@@ -142,16 +142,17 @@ struct C2POut {
 
 // Setup of the inversion (con2prim_robust.hpp:303-366).  Returns false when
 // the input is NaN (the reference returns failure before touching prims).
+// flr: the zone's entry of its view's floor table, or null.
 template <bool MINK>
 __device__ __forceinline__ bool c2p_setup(const Par &p, const Pt &g, const double U[PHX_NCONS],
                                           double x1, double x2, double x3, Residual &res,
                                           double rcon[3], double rcov[3], double bu[3],
-                                          double Bprim[3], double &bdotr) {
+                                          double Bprim[3], double &bdotr, const double2 *flr = nullptr) {
   if (is_nan(U[PHX_CRHO]) || is_nan(U[PHX_CMOM]) || is_nan(U[PHX_CENG])) return false;
   const double gdet = MINK ? 1.0 : g.detgam;
   const double igdet = MINK ? 1.0 : rcp_p(gdet);  // 1 / 1 = 1 in both builds
   double rhoflr = 0.0, epsflr;
-  const FloorPt fl = floor_point(p, x1, x2, x3);
+  const FloorPt fl = flr ? floor_load(flr) : floor_point(p, x1, x2, x3);
   floors_from(p, fl, rhoflr, epsflr);
   rhoflr *= p.fsf;
   const double gam_max = p.g0;

@@ -322,6 +322,11 @@ struct BView {
   double x0[3], dx[3];
   double *prim, *cons, *flux, *face_sig, *cell_sig, *fail, *src, *emf, *dudt;
   const double *gcent, *gface1, *gface2, *gderiv;
+  // floor_point's (r, s) at the n1t cell centres and then the n1t + 1 faces
+  // along X1, or null: a plan's views hold it where the floors depend on X1 alone
+  // and are not constant (two exponentials, 40 FP64 instructions, at every
+  // zone or face otherwise).
+  const double2 *flr;
   int fmks;
   __device__ __forceinline__ long long idx(int k, int j, int i) const {
     return ((long long)k * n2t + j) * n1t + i;
@@ -335,6 +340,17 @@ struct BView {
   __device__ __forceinline__ int ks() const { return ndim >= 3 ? ng : 0; }
   __device__ __forceinline__ int ke() const { return ndim >= 3 ? ng + nx3 - 1 : 0; }
 };
+
+// floor_point of the cell centre / X1 face i, from the view's table where it
+// has one (the same values: the table is floor_point's)
+__device__ __forceinline__ FloorPt floor_load(const double2 *t) {
+  const double2 v = __ldg(t);
+  return FloorPt{v.x, v.y};
+}
+__device__ __forceinline__ const double2 *floor_cell(const BView &b, int i) { return b.flr ? b.flr + i : nullptr; }
+__device__ __forceinline__ const double2 *floor_face1(const BView &b, int i) {
+  return b.flr ? b.flr + b.n1t + i : nullptr;
+}
 
 // ------------------------------------------------------------- geometry
 // Point geometry (values at a cell centre or a face).

@@ -128,6 +128,7 @@ __device__ __forceinline__ void floors_at(const Par &p, const BView &b, const Ra
   bool floor_applied = false;
   double drho = 0.0, du = 0.0, dprs = 0.0, dgm1 = 0.0, bp[3] = {0.0, 0.0, 0.0};
   double x1 = 0.0, x2 = 0.0, x3 = 0.0;
+  const double2 *flr = nullptr;
   if (valid) {
     for (int v = 0; v < PHX_NPRIM; v++) pr[v] = b.prim[v * vs + id];
     for (int m = 0; m < PHX_NCONS; m++) U[m] = b.cons[m * vs + id];
@@ -135,7 +136,8 @@ __device__ __forceinline__ void floors_at(const Par &p, const BView &b, const Ra
     x2 = b.Xc(1, j);
     x3 = b.Xc(2, k);
     double rho_floor, sie_floor;
-    get_floors(p, x1, x2, x3, rho_floor, sie_floor);
+    flr = floor_cell(b, i);
+    floors_from(p, flr ? floor_load(flr) : floor_point(p, x1, x2, x3), rho_floor, sie_floor);
     const double e_max = p.smax0;
     double rho_floor_max = rho_floor;
     double u_floor_max = rho_floor * sie_floor;
@@ -188,7 +190,7 @@ __device__ __forceinline__ void floors_at(const Par &p, const BView &b, const Ra
   Residual res;
   double rcon[3], rcov[3], bu[3], Bprim[3] = {0.0, 0.0, 0.0}, bdotr = 0.0;
   bool setup_ok = false;
-  if (valid && floor_applied) setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr);
+  if (valid && floor_applied) setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr, flr);
   C2POut out{0, 0, false, true, false};
   const double mu = regula_falsi_warp(p, res, setup_ok, 0.0, 1.0, valid ? pr[PHX_PMU] : 0.0, out);
   if (!valid) return;
@@ -271,6 +273,17 @@ void launch_floors(const Par &p, const BView &b, Range3 r, DevStats *stats, unsi
     k_floors<false><<<(unsigned)((n + T - 1) / T), T, 0, s>>>(p, b, r, n, stats, err, flag);
   else
     k_floors<true><<<(unsigned)((n + T - 1) / T), T, 0, s>>>(p, b, r, n, stats, err, flag);
+}
+
+__global__ void __launch_bounds__(128) k_floor_table(Par p, BView b, double2 *t) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= 2 * b.n1t + 1) return;
+  const FloorPt f = floor_point(p, q < b.n1t ? b.Xc(0, q) : b.Xf(0, q - b.n1t), 0.0, 0.0);
+  t[q] = make_double2(f.r, f.s);
+}
+
+void launch_floor_table(const Par &p, const BView &b, double2 *t, cudaStream_t s) {
+  k_floor_table<<<(2 * b.n1t + 1 + 127) / 128, 128, 0, s>>>(p, b, t);
 }
 
 // ------------------------------------------------------------- batched

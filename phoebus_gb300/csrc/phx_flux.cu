@@ -2,19 +2,22 @@
 // reconstruction + Riemann kernels, one launch per direction.
 //
 // The reference reconstructs every variable into ql/qr arrays (K1) and then
-// solves one Riemann problem per face (K2).  Here each face's two states are
-// produced and consumed in registers:
-//   X1: a CTA stages four (k, j) pencils' reconstructed primitive rows in
-//       shared memory with one tiled TMA copy per pencil
+// solves one Riemann problem per face (K2).  Here a thread produces and
+// consumes each face's two states:
+//   X1: a CTA stages one to four (k, j) pencils' primitive rows in shared
+//       memory with one tiled TMA copy per pencil
 //       (cp.async.bulk.tensor through a 5-D tensor map of the primitive
 //       array: i split in S rows of n1t/S, j, k, variable), completing on an
 //       mbarrier (1-D cp.async.bulk per row, or plain loads, where the block
 //       shape does not admit the map); lanes reconstruct consecutive cells and
 //       the left state of face i (the upper-face value of cell i-1) moves to
 //       lane i with __shfl_up_sync.
-//   X2, X3: a thread sweeps a segment of faces along the direction with the
-//       5-point stencil window and the previous cell's upper-face state held
-//       in registers; consecutive lanes are consecutive i (coalesced).
+//   X2, X3: a thread sweeps a segment of faces along the direction, one
+//       variable's stencil at a time; consecutive lanes are consecutive i
+//       (coalesced), and the cells a stencil shares with its neighbours come
+//       from L1.
+// The face states pass from the reconstruction to the Riemann solver through
+// shared memory (FaceStates).
 // Faces computed, per direction d: along d [s, e+1]; transverse active
 // directions [s-1, e+1].  These are all the faces FluxDivergence, FluxCT and
 // EstimateTimestep read.
@@ -46,8 +49,11 @@ __device__ __forceinline__ void face_flux(const Par &p, const BView &b, int k, i
     f.gammadet = f.g.detgam;
     f.gdd = f.g.gamcon[DIR][DIR];
   }
+  const double2 *flr = DIR == 0 ? floor_face1(b, i) : nullptr;
   if (col) {
     f.fl = *col;
+  } else if (flr) {
+    f.fl = floor_load(flr);
   } else {
     f.fl = floor_point(p, DIR == 0 ? b.Xf(0, i) : b.Xc(0, i), DIR == 1 ? b.Xf(1, j) : b.Xc(1, j),
                        DIR == 2 ? b.Xf(2, k) : b.Xc(2, k));
@@ -448,7 +454,7 @@ __device__ __forceinline__ void sweep_at(const Par &p, const BView &b, int alo, 
   // X2 and X3 faces of this column share X1 (= the cell centre of column a)
   FloorPt col{};
   const bool use_col = DIR != 0 && floors_x1_only(p);
-  if (use_col) col = floor_point(p, b.Xc(0, a), 0.0, 0.0);
+  if (use_col) col = b.flr ? floor_load(floor_cell(b, a)) : floor_point(p, b.Xc(0, a), 0.0, 0.0);
   // states: fs[0] and fs[1] the upper-face values of the previous and this
   // cell in turn, fs[2] the lower-face values of this cell
   int cur = 0;

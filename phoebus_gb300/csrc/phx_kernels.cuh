@@ -253,6 +253,8 @@ void launch_flux_sweep_batched(const Par &p, bool mink, int dir, const BView *vi
                                int nitems, int grid, int seg_target, cudaStream_t s);
 void launch_c2p_fixup_batched(const Par &p, bool mink, const BView *views, const WorkItem *items, int nitems,
                               cudaStream_t s);
+// floor_point at b's cell centres and X1 faces: t[2 n1t + 1] (BView::flr)
+void launch_floor_table(const Par &p, const BView &b, double2 *t, cudaStream_t s);
 void launch_floors_batched(const Par &p, bool mink, const BView *views, const WorkItem *items, int nitems,
                            DevStats *stats, unsigned int *err, cudaStream_t s);
 int x1_npencil(const BView &b);
