@@ -126,6 +126,7 @@ __device__ __forceinline__ void floors_at(const Par &p, const BView &b, const Ra
   }
   double pr[PHX_NPRIM], U[PHX_NCONS];
   bool floor_applied = false;
+  double W = 1.0;
   double drho = 0.0, du = 0.0, dprs = 0.0, dgm1 = 0.0, bp[3] = {0.0, 0.0, 0.0};
   double x1 = 0.0, x2 = 0.0, x3 = 0.0;
   const double2 *flr = nullptr;
@@ -141,6 +142,25 @@ __device__ __forceinline__ void floors_at(const Par &p, const BView &b, const Ra
     const double e_max = p.smax0;
     double rho_floor_max = rho_floor;
     double u_floor_max = rho_floor * sie_floor;
+#ifndef PHX_EXACT
+    // production build: v lowered once, W = (1 + v.v) rsqrt(1 + v.v), kept for
+    // the ceiling test, and b^2 without b^0 (its alpha cancels).  Within a few
+    // ulps of the ceiling W is the square root itself: con2prim puts zones
+    // onto the ceiling, and the ceiling's rescaling is not continuous there.
+    const double vp[3] = {pr[PHX_PVEL], pr[PHX_PVEL + 1], pr[PHX_PVEL + 2]};
+    double vlo[3] = {vp[0], vp[1], vp[2]};
+    if constexpr (!MINK) lower_sp(g, vp, vlo);
+    const double Wsq = 1. + dot3(vp, vlo), iW = rsqrt_p(Wsq);
+    const bool inside = dexp(Wsq) >= 16 && dexp(Wsq) <= 2030;
+    W = Wsq * iW;
+    const long long ulps = __double_as_longlong(W) - __double_as_longlong(p.g0);
+    if (!inside || (ulps < 16 && ulps > -16)) W = sqrt(Wsq);
+    if (p.enable_mhd_floors) {
+      const double bb[3] = {pr[PHX_PB], pr[PHX_PB + 1], pr[PHX_PB + 2]};
+      const double Bdotv = dot3(bb, vlo);
+      const double Bsq = dot_sp<MINK>(g, bb, bb);
+      const double bsq = inside ? fma(Bsq * iW, iW, Bdotv * Bdotv) : (Bsq + W * W * Bdotv * Bdotv) * iW * iW;
+#else
     if (p.enable_mhd_floors) {
       const double vp[3] = {pr[PHX_PVEL], pr[PHX_PVEL + 1], pr[PHX_PVEL + 2]};
       const double bb[3] = {pr[PHX_PB], pr[PHX_PB + 1], pr[PHX_PB + 2]};
@@ -162,13 +182,14 @@ __device__ __forceinline__ void floors_at(const Par &p, const BView &b, const Ra
       const double alpha = MINK ? 1.0 : g.alpha;
       const double bcon0 = div_p(W * Bdotv, alpha);
       const double bsq = (Bsq + alpha * alpha * bcon0 * bcon0) * iW * iW;
+#endif
       rho_floor_max = rmax(rho_floor_max, div_p(bsq, p.bsqorho0));
       u_floor_max = rmax(u_floor_max, div_p(bsq, p.bsqou0));
       rho_floor_max = rmax(rho_floor_max, div_p(rmax(pr[PHX_PENG], u_floor_max), e_max));
     }
     drho = rho_floor_max - pr[PHX_PRHO];
     du = u_floor_max - pr[PHX_PENG];
-    if (drho > 0. || du > 0.) {
+    if (gt(drho, 0.) || gt(du, 0.)) {
       floor_applied = true;
       drho = rmax(drho, du / sie_floor);
       du = rmax(du, sie_floor * drho);
@@ -228,8 +249,12 @@ __device__ __forceinline__ void floors_at(const Par &p, const BView &b, const Ra
   }
   const double gamma_max = p.g0, e_max = p.smax0;
   double vpcon[3] = {pr[PHX_PVEL], pr[PHX_PVEL + 1], pr[PHX_PVEL + 2]};
-  const double W = lorentz<MINK>(g, vpcon);
-  const bool ceiling_applied = (W > gamma_max || div_p(pr[PHX_PENG], pr[PHX_PRHO]) > e_max);
+#ifdef PHX_EXACT
+  W = lorentz<MINK>(g, vpcon);
+#else
+  if (floor_applied) W = lorentz<MINK>(g, vpcon);  // the velocity is new; else W stands
+#endif
+  const bool ceiling_applied = gt(W, gamma_max) || gt(div_p(pr[PHX_PENG], pr[PHX_PRHO]), e_max);
   if (ceiling_applied) {
     const double rescale = sqrt(gamma_max * gamma_max - 1.) / (W * W - 1.);
     for (int d = 0; d < 3; d++) {
