@@ -746,7 +746,7 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
   if (!(is > 0.0f && is < 1e3f)) return false;
   double x = f2d_bits(mp.h) + f2d_bits(mp.l);
   const float tol = d2f_bits(p.c2p_tol);
-  float f = 0.0f, gain = 1.0f;
+  float f = 0.0f;
   out.iterations = out.evals = 0;
 #pragma unroll 1
   for (;;) {
@@ -756,7 +756,6 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
     if (out.evals > 0 && fabsf(step) > 1e-9f * m) {  // secant through the last two evaluations
       const float isec = step * rcp_f32(f - fn);
       if (!(isec > 0.0f && isec < 1e3f)) return false;
-      gain = fabsf(is * rcp_f32(isec) - 1.0f) <= 0.03125f ? 16.0f : 1.0f;
       is = isec;
     }
     out.evals++;
@@ -765,8 +764,11 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
     step = f * is;
     if (!(fabsf(step) <= 0.5f * m)) return false;
     x -= f2d_bits(step);
-    // the error after this step: the step times the slope's relative error
-    if (fabsf(step) <= gain * tol) {
+    // The error after this step is the step times the slope's relative error.
+    // Two secants that agree say nothing about the slope beyond the root, where
+    // the residual has its kink (nua = nub, slopes up to 1.9 apart: an error
+    // below the step).
+    if (fabsf(step) <= tol) {
       mu = x < 1.0 ? x : 1.0;
       return x > 0.0;
     }

@@ -1,0 +1,75 @@
+"""The production build's con2prim root at the ends of the parameter range:
+fast and cold zones, whose residual changes slope at the root."""
+import numpy as np
+import pytest
+
+from phoebus_gb300 import abi
+from tests.util import host
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(a):
+    import torch
+
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def zone_prims(n, seed, gm1, Wmax, logsie=(-6.0, 1.0)):
+    """Log-uniform Lorentz factor in [1, Wmax] and u / rho, half the zones
+    magnetised with B^2 / rho log-uniform in [1e-4, 1e2]."""
+    rng = np.random.default_rng(seed)
+
+    def iso():
+        c, ph = rng.uniform(-1, 1, n), rng.uniform(0, 2 * np.pi, n)
+        s = np.sqrt(1 - c * c)
+        return np.stack([s * np.cos(ph), s * np.sin(ph), c])
+
+    rho, sie = 10.0 ** rng.uniform(-6, 0, n), 10.0 ** rng.uniform(*logsie, n)
+    W = Wmax ** rng.uniform(0, 1, n)
+    prim = np.zeros((abi.NPRIM, n))
+    prim[abi.PRHO], prim[abi.PENG], prim[abi.PPRS] = rho, rho * sie, gm1 * rho * sie
+    prim[abi.PVEL:abi.PVEL + 3] = np.sqrt(W * W - 1.0) * iso()
+    prim[abi.PB:abi.PB + 3] = np.sqrt(10.0 ** rng.uniform(-4, 2, n) * rho) * iso() * (np.arange(n) % 2)
+    prim[abi.PGM1], prim[abi.PTMP] = gm1 + 1.0, sie
+    return prim
+
+
+def solve(ctx, p, cons, prim0, learned=False):
+    """Primitives, fail flags and statistics of one call; an unbracketed root
+    raises."""
+    import torch
+
+    c, pr = dev(cons), dev(prim0)
+    fail = torch.zeros(cons.shape[1], dtype=torch.float64, device="cuda")
+    ctx.c2p_stats(reset=True)
+    ctx.ConservedToPrimitiveZones(p, c, pr, fail=fail, learned=learned)
+    ctx.check()
+    return host(pr), host(fail), host(c), ctx.c2p_stats(reset=True)
+
+
+def reference(oracle, p, cons, prim0):
+    c, pr, fail = cons.copy(), prim0.copy(), np.zeros(cons.shape[1])
+    assert oracle.ConservedToPrimitiveZones(p, c, pr, fail=fail) == 0
+    return pr, fail, c
+
+
+@pytest.mark.parametrize("gm1,tol,Wmax", [(2 / 3, 1e-9, 50.0), (2 / 3, 1e-10, 50.0), (1 / 3, 1e-10, 100.0),
+                                          (2 / 3, 1e-11, 100.0)])
+def test_fast_cold_zones_within_tolerance(ctx_fast, oracle, gm1, tol, Wmax):
+    """|mu - mu*| <= tol for every zone, mu* from the bracketed iteration at
+    tolerance 1e-15: its half width, and the residual's rounding of 1 - v^2
+    (2.2e-16 W^2 of 1 / W in mu = 1 / (h W): at most 2e-14 here) stay below
+    1e-13.  Half the zones are cold, half start 1% off the root."""
+    n = 400_000
+    p = abi.default_params(gm1=gm1, c2p_tol=tol, c2p_max_iter=100)
+    prim = zone_prims(n, int(1e3 * gm1 + Wmax), gm1, Wmax)
+    cons = oracle.PrimitiveToConservedZones(p, prim)
+    mu, _, _ = reference(oracle, abi.default_params(gm1=gm1, c2p_tol=1e-15, c2p_max_iter=200), cons, prim * 0.0)
+    mu = mu[abi.PMU]
+    prim0 = prim * 0.0
+    prim0[abi.PMU, ::2] = np.minimum(mu[::2] * (1.0 + 0.01 * np.sin(np.arange(n)[::2])), 1.0)
+    got, _, _, stats = solve(ctx_fast, p, cons, prim0)
+    over = np.abs(got[abi.PMU] - mu) > tol + 1e-13
+    assert not over.any(), (int(over.sum()), np.abs(got[abi.PMU] - mu).max() / tol)
+    assert stats["residual_evals"] < 2 * n  # the fast root is the one taken
