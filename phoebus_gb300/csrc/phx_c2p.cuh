@@ -656,7 +656,9 @@ struct FastResidual {
   }
   // false (the reference's expressions apply): a density small enough for the
   // reference's bound on h rho, an energy below 0, ExpX1RhoU's floor active
-  __device__ __forceinline__ bool eval64(const Par &p, const Residual &r, double mu, double &f) const {
+  // room: about the relative change of mu that switches the velocity bound or
+  // one of the energy bounds
+  __device__ __forceinline__ bool eval64(const Par &p, const Residual &r, double mu, double &f, float &room) const {
     const double x = rcp_p(fma(mu, r.bsq, 1.0));
     const double mr = mu * r.rbsq;
     const double rb = x * fma(x, r.rsq + mr, mr);
@@ -664,11 +666,15 @@ struct FastResidual {
     const double mrb = mu * rb;
     const double A = fma(-0.5 * r.bsq_rpsq, mux * mux, qh) - mrb;
     double v2 = mu * mrb;
+    const float dv = fabsf(d2f_bits(v2) - v0sq.h);
     if (gt_bits(v2, r.v0sq)) v2 = r.v0sq;
     const double om = 1.0 - v2;
     const double W = rsqrt_p(om), iW = om * W;
     double e = fma(W, A, W - 1.0);
     if (dexp(e) == 0x7ff) return false;  // NaN or infinity
+    const float ef = d2f_bits(e), Wf = d2f_bits(W);  // mu de/dmu is of size W (W (1 + e) + mrb + |A|)
+    const float de = Wf * fmaf(Wf, 1.0f + fabsf(ef), d2f_bits(mrb) + fabsf(d2f_bits(A)));
+    room = fminf(0.5f * dv, fminf(fabsf(ef - efl), fabsf(ef - emax)) * rcp_f32(de));
     if (!gt_bits(e, efl64)) {
       if (p.floor_type == PHX_FLOOR_EXPX1_RHO_U) return false;
       e = efl64;
@@ -713,7 +719,7 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
       }
     }
   }
-  float last = 1.0f;
+  float last = 1.0f, span = 1.0f;  // span: how far from the root the slope's points may lie
   for (int it = 0; it < 24; it++) {
     const float f = rf.eval(m, s);
     if (f > 0.0f)
@@ -724,6 +730,7 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
     if (!(n > lo && n < hi)) n = 0.5f * (lo + hi);
     const float d = fabsf(n - m);
     m = n;
+    span = d;
     // FP32 rounding reached: the step is at rounding level, or small and no longer shrinking
     if (d <= 1e-6f * m || (d <= 1e-3f * m && d > 0.5f * last)) break;
     last = d;
@@ -736,27 +743,37 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
 #pragma unroll 1
   for (int it = 0; it < 5; it++) {
     const float f = rf.evalp(mp);
-    if (it > 0 && fabsf(step) > 1e-7f * m) is = step * rcp_f32(fp - f);
+    if (it > 0 && fabsf(step) > 1e-7f * m) {
+      is = step * rcp_f32(fp - f);
+      span = fabsf(step);
+    }
     step = f * is;
     fp = f;
     if (!(fabsf(step) <= 0.5f * m)) return false;
+    if (it == 0) span += fabsf(step) + 2e-7f * m;
     mp = ff_addf(mp, -step);
     if (fabsf(step) <= 4e-12f * m) break;
   }
   if (!(is > 0.0f && is < 1e3f)) return false;
   double x = f2d_bits(mp.h) + f2d_bits(mp.l);
   const float tol = d2f_bits(p.c2p_tol);
+  const float tight = fmaxf(0.125f * tol, fminf(tol, 1e-12f * m));  // the residual's rounding is of that size
   float f = 0.0f;
   out.iterations = out.evals = 0;
 #pragma unroll 1
   for (;;) {
     double f64;
-    if (out.evals >= C2P_FAST_EVALS || !(x > 0.0 && x <= 1.0) || !rf.eval64(p, res, x, f64)) return false;
+    float room;
+    if (out.evals >= C2P_FAST_EVALS || !(x > 0.0 && x <= 1.0) || !rf.eval64(p, res, x, f64, room)) return false;
     const float fn = d2f_bits(f64);
-    if (out.evals > 0 && fabsf(step) > 1e-9f * m) {  // secant through the last two evaluations
+    if (out.evals > 0 && fabsf(step) > 1e-11f * m) {  // secant through the last two evaluations
       const float isec = step * rcp_f32(f - fn);
-      if (!(isec > 0.0f && isec < 1e3f)) return false;
-      is = isec;
+      if (isec > 0.0f && isec < 1e3f) {
+        is = isec;
+        span = fabsf(step);
+      } else if (fabsf(step) > 1e-9f * m) {
+        return false;
+      }
     }
     out.evals++;
     out.iterations++;
@@ -767,8 +784,10 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
     // The error after this step is the step times the slope's relative error.
     // Two secants that agree say nothing about the slope beyond the root, where
     // the residual has its kink (nua = nub, slopes up to 1.9 apart: an error
-    // below the step).
-    if (fabsf(step) <= tol) {
+    // below the step).  Where a bound switches within reach of the points the
+    // slope comes from, slopes up to 6 apart were seen: the step has to be an
+    // eighth of the tolerance.
+    if (fabsf(step) <= (room * m > 2.0f * span ? tol : tight)) {
       mu = x < 1.0 ? x : 1.0;
       return x > 0.0;
     }

@@ -1,5 +1,6 @@
 """The production build's con2prim root at the ends of the parameter range:
-fast and cold zones, whose residual changes slope at the root."""
+fast and cold zones, whose residual changes slope at the root, and bounds that
+switch beside it."""
 import numpy as np
 import pytest
 
@@ -73,3 +74,35 @@ def test_fast_cold_zones_within_tolerance(ctx_fast, oracle, gm1, tol, Wmax):
     over = np.abs(got[abi.PMU] - mu) > tol + 1e-13
     assert not over.any(), (int(over.sum()), np.abs(got[abi.PMU] - mu).max() / tol)
     assert stats["residual_evals"] < 2 * n  # the fast root is the one taken
+
+
+@pytest.mark.parametrize("tol", [1e-8, 1e-9, 1e-10])
+@pytest.mark.parametrize("bound", ["floor", "ceiling"])
+def test_bound_switching_beside_the_root(ctx_fast, oracle, tol, bound):
+    """Zones whose velocity is bounded (W = 5) and whose energy floor or ceiling
+    switches within 1e-9 to 1e-2 of the root, where the residual's slope changes
+    by several times.  From the root backwards, unmagnetised: with vt = mu r the
+    unbounded speed, mu = (1 - vt^2) / nu, nu = (1 + a)(1 + e) / W,
+    q = (1 + e) / W - 1 + vt r.  Bar as above."""
+    n, gm1, W = 200_000, 2.0 / 3.0, 5.0
+    rng = np.random.default_rng(41)
+    p = abi.default_params(gm1=gm1, c2p_tol=tol, c2p_max_iter=100)
+    p.enable_floors, p.rho0_floor, p.sie0_floor = 1, 1e-6, 1e-3
+    p.enable_ceilings, p.gam0_ceiling, p.sie0_ceiling = 1, W, 2.0
+    e = (1e-3 if bound == "floor" else 2.0) * (1.0 + 10.0 ** rng.uniform(-9, -2, n) * rng.choice([-1.0, 1.0], n))
+    vt = rng.uniform(np.sqrt(0.961), 0.999, n)
+    a = gm1 * e / (1.0 + e)
+    mu = (1.0 - vt * vt) / ((1.0 + a) * (1.0 + e) / W)
+    r = vt / mu
+    cons = np.zeros((abi.NCONS, n))
+    cons[abi.CRHO] = 10.0 ** rng.uniform(-3, 0, n)
+    cons[abi.CMOM] = r * cons[abi.CRHO]
+    cons[abi.CENG] = ((1.0 + e) / W - 1.0 + vt * r) * cons[abi.CRHO]
+    prim0 = np.zeros((abi.NPRIM, n))
+    pref = p.__class__.from_buffer_copy(p)
+    pref.c2p_tol, pref.c2p_max_iter = 1e-15, 200
+    ref, _, _ = reference(oracle, pref, cons, prim0)
+    prim0[abi.PMU, ::2] = np.minimum(ref[abi.PMU, ::2] * (1.0 + 0.01 * np.sin(np.arange(n)[::2])), 1.0)
+    got, _, _, _ = solve(ctx_fast, p, cons, prim0)
+    over = np.abs(got[abi.PMU] - ref[abi.PMU]) > tol + 1e-13
+    assert not over.any(), (int(over.sum()), np.abs(got[abi.PMU] - ref[abi.PMU]).max() / tol)
