@@ -106,3 +106,25 @@ def test_bound_switching_beside_the_root(ctx_fast, oracle, tol, bound):
     got, _, _, _ = solve(ctx_fast, p, cons, prim0)
     over = np.abs(got[abi.PMU] - ref[abi.PMU]) > tol + 1e-13
     assert not over.any(), (int(over.sum()), np.abs(got[abi.PMU] - ref[abi.PMU]).max() / tol)
+
+
+@pytest.mark.parametrize("floor", [0.0, 1e-18])
+@pytest.mark.parametrize("sign_tau", [1.0, -1.0])
+def test_negative_density(ctx_fast, oracle, floor, sign_tau):
+    """D < 0 (an update that overshot): the density is the floor, and where
+    that is below the reference's bound on h rho the residual no longer is the
+    one of the ideal gas.  Same root and same fail flags as the reference; hydro
+    (sqrt(D) divides the field)."""
+    n, tol = 4000, 1e-10
+    p = abi.default_params(gm1=1 / 3, c2p_tol=tol, c2p_max_iter=100, mhd=0)
+    prim = zone_prims(n, 31, 1 / 3, 20.0)
+    prim[abi.PB:abi.PB + 3] = 0.0
+    cons = oracle.PrimitiveToConservedZones(p, prim)
+    cons[abi.CRHO] *= -1.0
+    cons[abi.CENG] *= sign_tau
+    p.enable_floors, p.rho0_floor, p.sie0_floor = int(floor > 0), floor, floor
+    ref, rfail, _ = reference(oracle, p, cons, prim * 0.0)
+    got, fail, _, _ = solve(ctx_fast, p, cons, prim * 0.0)
+    assert np.array_equal(fail, rfail)
+    assert np.array_equal(np.isnan(got[abi.PMU]), np.isnan(ref[abi.PMU]))
+    assert np.nanmax(np.abs(got[abi.PMU] - ref[abi.PMU])) <= 2.0 * tol + 1e-13
