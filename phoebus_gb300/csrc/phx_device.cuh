@@ -27,7 +27,8 @@ constexpr double kDBLMAX = 1.7976931348623157e308;
 // Comparisons of doubles on the integer pipe (an FP64 comparison holds the
 // FP64 pipe like an FMA): order_bits is increasing in x (-0 below +0, NaN
 // with a clear sign bit on top).  max_num / min_num return the other operand
-// where one is NaN, as fmax / fmin do.
+// where one is NaN, as fmax / fmin do.  gt_bits takes +0 above -0; where that
+// matters, gt below compares as the IEEE > does.
 __device__ __forceinline__ long long order_bits(double x) {
   const long long b = __double_as_longlong(x);
   return b ^ ((b >> 63) & 0x7fffffffffffffffll);
@@ -36,6 +37,11 @@ __device__ __forceinline__ double from_order_bits(long long k) {
   return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
 }
 __device__ __forceinline__ bool gt_bits(double a, double b) { return order_bits(a) > order_bits(b); }
+// order_bits with -0 equal to +0
+__device__ __forceinline__ long long value_bits(double x) {
+  const long long b = __double_as_longlong(x);
+  return b >= 0 ? b : (long long)(0x8000000000000000ull - (unsigned long long)b);
+}
 __device__ __forceinline__ bool nan_bits(double x) {
   return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
 }
@@ -75,12 +81,12 @@ __device__ __forceinline__ double clamp0(double x) {
   return b <= 0x7ff0000000000000ll && b > 0 ? x : 0.0;
 #endif
 }
-// a > b (false where either is NaN)
+// a > b (false where either is NaN, and for two zeros of any sign)
 __device__ __forceinline__ bool gt(double a, double b) {
 #ifdef PHX_EXACT
   return a > b;
 #else
-  return gt_bits(a, b) && !nan_bits(a) && !nan_bits(b);
+  return value_bits(a) > value_bits(b) && !nan_bits(a) && !nan_bits(b);
 #endif
 }
 __device__ __forceinline__ bool is_nan(double x) {
