@@ -472,15 +472,21 @@ struct Closure {
   // athin of the closure at xi: (3 closure_fn - 1) / 2 = xi^2 (2 xi - 1)
   __device__ __forceinline__ static double athin_of(double xi) { return xi * xi * fma(2.0, xi, -1.0); }
   // 1 / sqrt(m2) of the rest-frame flux's squared magnitude and xi = H / J
-  // bounded to [0, 1]; a vanishing flux has no direction: both 0 (the
-  // reference's f = H / (H + SMALL)), NaN otherwise
+  // bounded to [0, 1]; a flux of 0 has no direction: both 0 (the reference's
+  // f = H / (H + SMALL)), NaN for a negative m2.  Magnitudes outside rsqrt_nr's
+  // range (H below 2.7e-152 or above 1e151) take the IEEE square root: J may be of
+  // that size.
   __device__ __forceinline__ static void flux_xi(double m2, double J, double &im, double &xi) {
     const int e = __double2hiint(m2) >> 20;
     if (e >= 16 && e <= 2030) {
       im = rsqrt_nr(m2);
       xi = smax(smin(1.0, ratio_p(m2 * im, J)), 0.0);
+    } else if (__double_as_longlong(m2) > 0) {
+      const double h = sqrt(m2);
+      im = 1.0 / h;
+      xi = smax(smin(1.0, ratio_p(h, J)), 0.0);
     } else {
-      im = xi = e >= 0 && e < 16 ? 0.0 : __longlong_as_double(0x7ff8000000000000ll);
+      im = xi = __double_as_longlong(m2) == 0 ? 0.0 : __longlong_as_double(0x7ff8000000000000ll);
     }
   }
   __device__ __forceinline__ void tilpi_from_prim(double J, const V3 &H, PiC &Pi) const {
@@ -1034,7 +1040,7 @@ __device__ __forceinline__ void face_state(const Closure<true, true> &c, double 
   double im, xi;
   c.flux_xi(ccov(H, H) - vH * vH, J, im, xi);
   const double Ja = J * c.athin_of(xi);
-  const double q = Ja * (im * im), qvH = q * vH;
+  const double q = (Ja * im) * im, qvH = q * vH;  // im^2 may overflow where H is tiny
   const double w3 = Ja * D3(fma(c.W2, c.v2raw, 1.0));
   const double a43 = D3(4 * c.W2) * J;
   const double vvPi = fma(qvH, vH, -w3 * c.v2raw);
