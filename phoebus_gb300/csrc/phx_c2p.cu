@@ -116,11 +116,13 @@ void launch_p2c_zones(const Par &p, long long n, const double *prim, const doubl
 // network out of the root-find kernel keeps that kernel's instruction
 // footprint small (fused, the two codes thrashed the instruction cache).
 constexpr int C2P_THREADS = 128;
-// Resident CTAs per SM the root-find kernels' registers are bounded for.
+// Resident CTAs per SM the root-find kernels' registers are bounded for; fast:
+// the kernel with the production root.
+constexpr int c2p_minb(bool mink, bool fast) { return !fast ? 1 : mink ? 4 : 3; }
 #ifdef PHX_EXACT
-constexpr int c2p_minb(bool) { return 1; }
+constexpr bool kC2PFast = false;
 #else
-constexpr int c2p_minb(bool mink) { return mink ? 4 : 3; }
+constexpr bool kC2PFast = true;
 #endif
 
 // Zones of a block index box.
@@ -323,11 +325,11 @@ __device__ __forceinline__ bool c2p_complete(const Par &p, const Z &zones, long 
   return success;
 }
 
-// Zones left to the retry launch: chunk offset and, in the exact build (whose
-// first kernel stops at an iteration cap), the saved RFState (it, evals, b1, b2
-// in 16/16/14/14 bits, then the sign and learned bits).  The production
-// build's list holds the zones its fast root did not accept, which start
-// again from the reference's bracket.
+// Zones left to the retry launch: chunk offset and, without the fast root
+// (where the first kernel stops at an iteration cap), the saved RFState (it,
+// evals, b1, b2 in 16/16/14/14 bits, then the sign and learned bits).  With the
+// fast root the list holds the zones it did not accept, which start again
+// from the reference's bracket.
 struct RetryBuf {
   int *count;
   int *idx;
@@ -351,13 +353,14 @@ __device__ __forceinline__ void rf_unpack(unsigned long long w, RFState &s) {
 }
 
 // con2prim of zones t0 .. t0 + count - 1, one zone per thread.  LEARNED:
-// the start bracket of zone t is brk[c * count + t - t0].  Zones that the fast
-// root does not accept (exact build: lanes that have not converged after cap
-// iterations, with their saved state) are appended to rb (warp-aggregated)
-// and left to k_c2p_retry, so that one slow zone does not hold 31 finished
-// lanes of its warp.
-template <class Z, bool MINK, bool LEARNED>
-__global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK)) k_c2p(Par p, Z zones, long long t0, long long count,
+// the start bracket of zone t is brk[c * count + t - t0].  FAST: the production
+// root; the exact build, and settings outside its rule (c2p_fast_allowed), take
+// the reference's iteration.  Zones that the fast root does not accept
+// (without FAST: lanes that have not converged after cap iterations, with their
+// saved state) are appended to rb (warp-aggregated) and left to k_c2p_retry, so
+// that one slow zone does not hold 31 finished lanes of its warp.
+template <class Z, bool MINK, bool LEARNED, bool FAST>
+__global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, FAST)) k_c2p(Par p, Z zones, long long t0, long long count,
                                                       const double *brk, int cap, RetryBuf rb, DevStats *stats,
                                                       unsigned int *err) {
   __shared__ unsigned int s_hist[PHX_C2P_HIST];
@@ -391,15 +394,18 @@ __global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK)) k_c2p(Par p, Z zo
     }
   }
   C2POut out{0, 0, false, true, false, false};
-#ifdef PHX_EXACT
   RFState st;
-  rf_start<LEARNED>(p, res, run, 0.0, 1.0, guess, lb, st);
-  rf_iterate(p, res, run, st, cap);
-  const bool defer = run && rf_running(p, st);
-#else
   double mu = guess;
-  const bool defer = run && !(c2p_fast_allowed(p) && c2p_fast_root<LEARNED>(p, res, guess, lb, mu, out));
+  bool defer;
+  if constexpr (FAST) {
+#ifndef PHX_EXACT
+    defer = run && !c2p_fast_root<LEARNED>(p, res, guess, lb, mu, out);
 #endif
+  } else {
+    rf_start<LEARNED>(p, res, run, 0.0, 1.0, guess, lb, st);
+    rf_iterate(p, res, run, st, cap);
+    defer = run && rf_running(p, st);
+  }
   const unsigned m = __ballot_sync(0xffffffffu, defer);
   if (m) {
     const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
@@ -409,20 +415,18 @@ __global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK)) k_c2p(Par p, Z zo
     if (defer) {
       const int pos = base + __popc(m & ((1u << lane) - 1u));
       rb.idx[pos] = (int)q;
-#ifdef PHX_EXACT
-      rb.a[pos] = st.a;
-      rb.b[pos] = st.b;
-      rb.ya[pos] = st.ya;
-      rb.yb[pos] = st.yb;
-      rb.packed[pos] = rf_pack(st);
-#endif
+      if constexpr (!FAST) {
+        rb.a[pos] = st.a;
+        rb.b[pos] = st.b;
+        rb.ya[pos] = st.ya;
+        rb.yb[pos] = st.yb;
+        rb.packed[pos] = rf_pack(st);
+      }
     }
   }
   bool success = false;
   if (valid && !defer) {
-#ifdef PHX_EXACT
-    const double mu = rf_result(st, guess, out);
-#endif
+    if constexpr (!FAST) mu = rf_result(st, guess, out);
     success = c2p_complete<Z, MINK>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, err);
   }
   if (stats) c2p_tally(s_hist, s_cnt, valid && !defer, out, setup_ok, success);
@@ -430,8 +434,9 @@ __global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK)) k_c2p(Par p, Z zo
 }
 
 // The deferred zones of a chunk: reload, set up again (the same
-// deterministic setup), restore the root-find state and iterate to the end.
-template <class Z, bool MINK>
+// deterministic setup), restore the root-find state (FAST: start the
+// reference's iteration) and iterate to the end.
+template <class Z, bool MINK, bool FAST>
 __global__ void __launch_bounds__(C2P_THREADS) k_c2p_retry(Par p, Z zones, long long t0, RetryBuf rb, DevStats *stats,
                                                             unsigned int *err) {
   __shared__ unsigned int s_hist[PHX_C2P_HIST];
@@ -457,17 +462,15 @@ __global__ void __launch_bounds__(C2P_THREADS) k_c2p_retry(Par p, Z zones, long 
       const double2 *flr;
       zones.template load<MINK>(t0 + rb.idx[k], id, g, U, x1, x2, x3, guess, flr);
       setup_ok = c2p_setup<MINK>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr, flr);
-#ifdef PHX_EXACT
-      st.a = rb.a[k];
-      st.b = rb.b[k];
-      st.ya = rb.ya[k];
-      st.yb = rb.yb[k];
-      rf_unpack(rb.packed[k], st);
-#endif
+      if constexpr (!FAST) {
+        st.a = rb.a[k];
+        st.b = rb.b[k];
+        st.ya = rb.ya[k];
+        st.yb = rb.yb[k];
+        rf_unpack(rb.packed[k], st);
+      }
     }
-#ifndef PHX_EXACT  // the fast root was not accepted: the reference's iteration from its start
-    rf_start<false>(p, res, valid && setup_ok, 0.0, 1.0, guess, nullptr, st);
-#endif
+    if constexpr (FAST) rf_start<false>(p, res, valid && setup_ok, 0.0, 1.0, guess, nullptr, st);
     rf_iterate(p, res, valid && setup_ok, st, p.c2p_max_iter);
     C2POut out{0, 0, false, true, false, false};
     bool success = false;
@@ -496,9 +499,8 @@ static void launch_bracket_any(const Par &p, const Z &z, long long t0, long long
 }
 
 // Zones per chunk of C2P_CHUNK; per chunk: [bracket launch], root-find
-// launch, retry launch over the deferred zones.  In the exact build the
-// root-find launch has an iteration cap (the production build's fast root ends
-// by itself and takes none); the
+// launch, retry launch over the deferred zones.  Without the fast root (which
+// ends by itself) the root-find launch has an iteration cap; the
 // caps default to a little above the mean iteration count of each start on
 // Kerr-Schild zones at tolerance 1e-10; PHX_C2P_CAP_PLAIN /
 // PHX_C2P_CAP_LEARNED in the environment override them (read once).
@@ -508,10 +510,9 @@ static int cap_from_env(const char *name, int dflt) {
   return c > 0 ? c : dflt;
 }
 
-template <class Z, bool MINK>
-static void launch_c2p_any(const Par &p, const Z &z, long long n, const MlpPacked *mlp, const C2PScratch &scr,
-                           DevStats *stats, unsigned int *err, cudaStream_t s) {
-  if (n <= 0) return;
+template <class Z, bool MINK, bool FAST>
+static void launch_c2p_root(const Par &p, const Z &z, long long n, const MlpPacked *mlp, const C2PScratch &scr,
+                            DevStats *stats, unsigned int *err, cudaStream_t s) {
   static const int cap_plain = cap_from_env("PHX_C2P_CAP_PLAIN", 12);
   static const int cap_learned = cap_from_env("PHX_C2P_CAP_LEARNED", 6);
   const int cap = mlp ? cap_learned : cap_plain;
@@ -523,12 +524,26 @@ static void launch_c2p_any(const Par &p, const Z &z, long long n, const MlpPacke
     cudaMemsetAsync(scr.count, 0, sizeof(int), s);
     if (mlp) {
       launch_bracket_any<Z, MINK>(p, z, t0, m, mlp, scr.brk, err, s);
-      k_c2p<Z, MINK, true><<<(unsigned)grid, C2P_THREADS, 0, s>>>(p, z, t0, m, scr.brk, cap, rb, stats, err);
+      k_c2p<Z, MINK, true, FAST><<<(unsigned)grid, C2P_THREADS, 0, s>>>(p, z, t0, m, scr.brk, cap, rb, stats, err);
     } else {
-      k_c2p<Z, MINK, false><<<(unsigned)grid, C2P_THREADS, 0, s>>>(p, z, t0, m, nullptr, cap, rb, stats, err);
+      k_c2p<Z, MINK, false, FAST><<<(unsigned)grid, C2P_THREADS, 0, s>>>(p, z, t0, m, nullptr, cap, rb, stats, err);
     }
-    k_c2p_retry<Z, MINK><<<retry_grid, C2P_THREADS, 0, s>>>(p, z, t0, rb, stats, err);
+    k_c2p_retry<Z, MINK, FAST><<<retry_grid, C2P_THREADS, 0, s>>>(p, z, t0, rb, stats, err);
   }
+}
+
+// Tolerances and iteration caps outside the fast root's rule keep kernels of
+// their own: with every zone of the fast kernel left to the retry launch, 1e6
+// Kerr-Schild zones at tolerance 2e-3 took 2.71 ms (capped iteration: 1.78 ms), at
+// 1e-16 3.29 ms (2.10), and the learned start was lost.
+template <class Z, bool MINK>
+static void launch_c2p_any(const Par &p, const Z &z, long long n, const MlpPacked *mlp, const C2PScratch &scr,
+                           DevStats *stats, unsigned int *err, cudaStream_t s) {
+  if (n <= 0) return;
+  if (kC2PFast && c2p_fast_allowed(p))
+    launch_c2p_root<Z, MINK, kC2PFast>(p, z, n, mlp, scr, stats, err, s);
+  else
+    launch_c2p_root<Z, MINK, false>(p, z, n, mlp, scr, stats, err, s);
 }
 
 void launch_c2p(const Par &p, const BView &b, Range3 r, DevStats *stats, unsigned int *err,
@@ -628,7 +643,7 @@ __global__ void __launch_bounds__(C2P_THREADS) kb_mlp_bracket(Par p, const BView
 // so warm zones (all of them once a run is under way) go through exactly the
 // plain kernel's code.
 template <bool MINK, bool LEARNED>
-__global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK)) kb_c2p(Par p, const BView *views, const WorkItem *items, int nitems,
+__global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, kC2PFast)) kb_c2p(Par p, const BView *views, const WorkItem *items, int nitems,
                                                        double *brk, DevStats *stats, unsigned int *err, int only) {
   if (only == 2 && *reinterpret_cast<const unsigned long long *>(brk + 4 * (long long)nitems * C2P_THREADS) == 0)
     return;  // no cold zone

@@ -460,6 +460,14 @@ __device__ __forceinline__ double regula_falsi_warp(const Par &p, Residual &res,
   return rf_result(s, guess, out);
 }
 
+// Largest number of FP64 evaluations of the production root before a zone takes
+// the reference's iteration; iteration caps below it keep the reference's own
+// counting.
+constexpr int C2P_FAST_EVALS = 5;
+__host__ __device__ __forceinline__ bool c2p_fast_allowed(const Par &p) {
+  return p.c2p_max_iter >= C2P_FAST_EVALS && p.c2p_tol >= 1e-15 && p.c2p_tol <= 1e-3;
+}
+
 #ifndef PHX_EXACT
 // ------------------------------------------------ production root find
 // The residual is FP64-bound: an FP64 instruction holds a sub-partition's
@@ -691,13 +699,6 @@ struct FastResidual {
   }
 };
 
-// Largest number of FP64 evaluations before a zone takes the reference's
-// iteration; iteration caps below it keep the reference's own counting.
-constexpr int C2P_FAST_EVALS = 5;
-__device__ __forceinline__ bool c2p_fast_allowed(const Par &p) {
-  return p.c2p_max_iter >= C2P_FAST_EVALS && p.c2p_tol >= 1e-15 && p.c2p_tol <= 1e-3;
-}
-
 // mu of one zone from its guess (> 0: a previous solution) or, LEARNED, the
 // predicted root lb[0] of a cold zone.  False: not accepted.  mu lies within
 // c2p_tol of the root where true, as the reference's final bracket has it.
@@ -797,8 +798,11 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
 
 // The reference's iteration for the zones the fast root leaves, kept out of
 // the callers' instruction stream.
-static __device__ __noinline__ double c2p_slow_root(const Par &p, Residual res, bool need, double guess, C2POut *out) {
-  return regula_falsi_warp<false>(p, res, need, 0.0, 1.0, guess, *out);
+template <bool LEARNED>
+static __device__ __noinline__ double c2p_slow_root(const Par &p, Residual res, bool need, double guess, double lb0,
+                                                    double lb1, double lb2, C2POut *out) {
+  const double lb[3] = {lb0, lb1, lb2};
+  return regula_falsi_warp<LEARNED>(p, res, need, 0.0, 1.0, guess, *out, lb);
 }
 #endif
 
@@ -813,12 +817,16 @@ __device__ __forceinline__ double c2p_root_warp(const Par &p, Residual &res, boo
   if (valid && c2p_fast_allowed(p)) need = !c2p_fast_root<LEARNED>(p, res, guess, lb, mu, out);
   if (!__any_sync(0xffffffffu, need)) return mu;
   C2POut slow{0, 0, false, true, false, false};
-  const double ms = c2p_slow_root(p, res, need, guess, &slow);
+  double ms;
+  if constexpr (LEARNED)
+    ms = c2p_slow_root<true>(p, res, need, guess, lb[0], lb[1], lb[2], &slow);
+  else
+    ms = c2p_slow_root<false>(p, res, need, guess, 0.0, 0.0, 0.0, &slow);
   if (need) {
     out.iterations = slow.iterations;
     out.evals = slow.evals;
     out.bracketed = slow.bracketed;
-    out.learned = false;
+    out.learned = slow.learned;
     mu = ms;
   }
   return mu;

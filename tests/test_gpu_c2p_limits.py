@@ -128,3 +128,25 @@ def test_negative_density(ctx_fast, oracle, floor, sign_tau):
     assert np.array_equal(fail, rfail)
     assert np.array_equal(np.isnan(got[abi.PMU]), np.isnan(ref[abi.PMU]))
     assert np.nanmax(np.abs(got[abi.PMU] - ref[abi.PMU])) <= 2.0 * tol + 1e-13
+
+
+@pytest.mark.parametrize("tol,max_iter", [(2e-3, 100), (1e-16, 100), (1e-10, 4)])
+@pytest.mark.parametrize("n", [129, 5000])
+def test_learned_start_outside_the_fast_rule(ctx_fast, oracle, tol, max_iter, n):
+    """Tolerances and iteration caps outside the fast rule keep the reference's
+    iteration, the learned start included: a network whose output is constant
+    (mu = e^-1, bracket e^-4 to 1) brackets every root in between."""
+    p = abi.default_params(gm1=1 / 3, c2p_tol=tol, c2p_max_iter=max_iter)
+    prim = zone_prims(n, 33, 1 / 3, 8.0, (-5.0, 0.0))
+    cons = oracle.PrimitiveToConservedZones(p, prim)
+    theta = np.zeros(abi.MLP_NPARAM, dtype=np.float32)
+    theta[-2:] = [-1.0, 0.0]
+    ctx_fast.mlp_set_weights(theta)
+    mu, _, _ = reference(oracle, abi.default_params(gm1=1 / 3, c2p_tol=1e-15, c2p_max_iter=200), cons, prim * 0.0)
+    mu = mu[abi.PMU]
+    inside = (mu > 1.02 * np.exp(-4.0)) & (mu < 0.98)  # the network's output has BF16 weights
+    got, _, _, stats = solve(ctx_fast, p, cons, prim * 0.0, learned=True)
+    assert inside.sum() > 0.9 * n and inside.sum() <= stats["learned_accepted"] <= n
+    assert stats["residual_evals"] >= 3 * n  # no zone by the fast root
+    if max_iter == 100:
+        assert np.abs(got[abi.PMU] - mu).max() <= tol + 1e-13
