@@ -119,11 +119,16 @@ constexpr int C2P_THREADS = 128;
 // Resident CTAs per SM the root-find kernels' registers are bounded for; fast:
 // the kernel with the production root.
 constexpr int c2p_minb(bool mink, bool fast) { return !fast ? 1 : mink ? 4 : 3; }
+// The root find of a kernel: the reference's iteration (the exact build, and
+// settings outside the fast root's rule), the production build's fast root, and
+// the fast root with an energy floor that follows the density.
+enum C2PRoot { C2P_REF, C2P_FAST, C2P_FAST_RHOU };
 #ifdef PHX_EXACT
 constexpr bool kC2PFast = false;
 #else
 constexpr bool kC2PFast = true;
 #endif
+static bool c2p_rhou(const Par &p) { return kC2PFast && p.floor_type == PHX_FLOOR_EXPX1_RHO_U; }
 
 // Zones of a block index box.
 struct BoxZones {
@@ -353,14 +358,13 @@ __device__ __forceinline__ void rf_unpack(unsigned long long w, RFState &s) {
 }
 
 // con2prim of zones t0 .. t0 + count - 1, one zone per thread.  LEARNED:
-// the start bracket of zone t is brk[c * count + t - t0].  FAST: the production
-// root; the exact build, and settings outside its rule (c2p_fast_allowed), take
-// the reference's iteration.  Zones that the fast root does not accept
-// (without FAST: lanes that have not converged after cap iterations, with their
-// saved state) are appended to rb (warp-aggregated) and left to k_c2p_retry, so
-// that one slow zone does not hold 31 finished lanes of its warp.
-template <class Z, bool MINK, bool LEARNED, bool FAST>
-__global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, FAST)) k_c2p(Par p, Z zones, long long t0, long long count,
+// the start bracket of zone t is brk[c * count + t - t0].  Zones that the fast
+// root does not accept (with C2P_REF: lanes that have not converged after cap
+// iterations, with their saved state) are appended to rb (warp-aggregated) and
+// left to k_c2p_retry, so that one slow zone does not hold 31 finished lanes of
+// its warp.
+template <class Z, bool MINK, bool LEARNED, C2PRoot ROOT>
+__global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, ROOT != C2P_REF)) k_c2p(Par p, Z zones, long long t0, long long count,
                                                       const double *brk, int cap, RetryBuf rb, DevStats *stats,
                                                       unsigned int *err) {
   __shared__ unsigned int s_hist[PHX_C2P_HIST];
@@ -397,9 +401,9 @@ __global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, FAST)) k_c2p(Par p
   RFState st;
   double mu = guess;
   bool defer;
-  if constexpr (FAST) {
+  if constexpr (ROOT != C2P_REF) {
 #ifndef PHX_EXACT
-    defer = run && !c2p_fast_root<LEARNED>(p, res, guess, lb, mu, out);
+    defer = run && !c2p_fast_root<LEARNED, ROOT == C2P_FAST_RHOU>(p, res, guess, lb, mu, out);
 #endif
   } else {
     rf_start<LEARNED>(p, res, run, 0.0, 1.0, guess, lb, st);
@@ -415,7 +419,7 @@ __global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, FAST)) k_c2p(Par p
     if (defer) {
       const int pos = base + __popc(m & ((1u << lane) - 1u));
       rb.idx[pos] = (int)q;
-      if constexpr (!FAST) {
+      if constexpr (ROOT == C2P_REF) {
         rb.a[pos] = st.a;
         rb.b[pos] = st.b;
         rb.ya[pos] = st.ya;
@@ -426,7 +430,7 @@ __global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, FAST)) k_c2p(Par p
   }
   bool success = false;
   if (valid && !defer) {
-    if constexpr (!FAST) mu = rf_result(st, guess, out);
+    if constexpr (ROOT == C2P_REF) mu = rf_result(st, guess, out);
     success = c2p_complete<Z, MINK>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, err);
   }
   if (stats) c2p_tally(s_hist, s_cnt, valid && !defer, out, setup_ok, success);
@@ -510,7 +514,7 @@ static int cap_from_env(const char *name, int dflt) {
   return c > 0 ? c : dflt;
 }
 
-template <class Z, bool MINK, bool FAST>
+template <class Z, bool MINK, C2PRoot ROOT>
 static void launch_c2p_root(const Par &p, const Z &z, long long n, const MlpPacked *mlp, const C2PScratch &scr,
                             DevStats *stats, unsigned int *err, cudaStream_t s) {
   static const int cap_plain = cap_from_env("PHX_C2P_CAP_PLAIN", 12);
@@ -524,26 +528,30 @@ static void launch_c2p_root(const Par &p, const Z &z, long long n, const MlpPack
     cudaMemsetAsync(scr.count, 0, sizeof(int), s);
     if (mlp) {
       launch_bracket_any<Z, MINK>(p, z, t0, m, mlp, scr.brk, err, s);
-      k_c2p<Z, MINK, true, FAST><<<(unsigned)grid, C2P_THREADS, 0, s>>>(p, z, t0, m, scr.brk, cap, rb, stats, err);
+      k_c2p<Z, MINK, true, ROOT><<<(unsigned)grid, C2P_THREADS, 0, s>>>(p, z, t0, m, scr.brk, cap, rb, stats, err);
     } else {
-      k_c2p<Z, MINK, false, FAST><<<(unsigned)grid, C2P_THREADS, 0, s>>>(p, z, t0, m, nullptr, cap, rb, stats, err);
+      k_c2p<Z, MINK, false, ROOT><<<(unsigned)grid, C2P_THREADS, 0, s>>>(p, z, t0, m, nullptr, cap, rb, stats, err);
     }
-    k_c2p_retry<Z, MINK, FAST><<<retry_grid, C2P_THREADS, 0, s>>>(p, z, t0, rb, stats, err);
+    k_c2p_retry<Z, MINK, ROOT != C2P_REF><<<retry_grid, C2P_THREADS, 0, s>>>(p, z, t0, rb, stats, err);
   }
 }
 
 // Tolerances and iteration caps outside the fast root's rule keep kernels of
 // their own: with every zone of the fast kernel left to the retry launch, 1e6
 // Kerr-Schild zones at tolerance 2e-3 took 2.71 ms (capped iteration: 1.78 ms), at
-// 1e-16 3.29 ms (2.10), and the learned start was lost.
+// 1e-16 3.29 ms (2.10), and the learned start was lost.  ExpX1RhoU's floor has
+// one too: left to the retry launch wherever the energy lies below that floor's
+// largest value, the same zones took 3.24 ms (1.04 with it).
 template <class Z, bool MINK>
 static void launch_c2p_any(const Par &p, const Z &z, long long n, const MlpPacked *mlp, const C2PScratch &scr,
                            DevStats *stats, unsigned int *err, cudaStream_t s) {
   if (n <= 0) return;
-  if (kC2PFast && c2p_fast_allowed(p))
-    launch_c2p_root<Z, MINK, kC2PFast>(p, z, n, mlp, scr, stats, err, s);
+  if (!kC2PFast || !c2p_fast_allowed(p))
+    launch_c2p_root<Z, MINK, C2P_REF>(p, z, n, mlp, scr, stats, err, s);
+  else if (c2p_rhou(p))
+    launch_c2p_root<Z, MINK, kC2PFast ? C2P_FAST_RHOU : C2P_REF>(p, z, n, mlp, scr, stats, err, s);
   else
-    launch_c2p_root<Z, MINK, false>(p, z, n, mlp, scr, stats, err, s);
+    launch_c2p_root<Z, MINK, kC2PFast ? C2P_FAST : C2P_REF>(p, z, n, mlp, scr, stats, err, s);
 }
 
 void launch_c2p(const Par &p, const BView &b, Range3 r, DevStats *stats, unsigned int *err,
@@ -642,9 +650,10 @@ __global__ void __launch_bounds__(C2P_THREADS) kb_mlp_bracket(Par p, const BView
 // plain kernel over the warm zones and the learned one over the cold zones,
 // so warm zones (all of them once a run is under way) go through exactly the
 // plain kernel's code.
-template <bool MINK, bool LEARNED>
-__global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, kC2PFast)) kb_c2p(Par p, const BView *views, const WorkItem *items, int nitems,
-                                                       double *brk, DevStats *stats, unsigned int *err, int only) {
+template <bool MINK, bool LEARNED, bool RHOU>
+__global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, kC2PFast))
+    kb_c2p(Par p, const BView *views, const WorkItem *items, int nitems, double *brk, DevStats *stats,
+           unsigned int *err, int only) {
   if (only == 2 && *reinterpret_cast<const unsigned long long *>(brk + 4 * (long long)nitems * C2P_THREADS) == 0)
     return;  // no cold zone
   __shared__ unsigned int s_hist[PHX_C2P_HIST];
@@ -696,7 +705,7 @@ __global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, kC2PFast)) kb_c2p(
       }
     }
     C2POut out{0, 0, false, true, false, false};
-    const double mu = c2p_root_warp<LEARNED>(p, res, valid && setup_ok, guess, out, lb);
+    const double mu = c2p_root_warp<LEARNED, RHOU>(p, res, valid && setup_ok, guess, out, lb);
     bool success = false;
     if (valid)
       success = c2p_complete<BoxZones, MINK>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, err);
@@ -705,22 +714,22 @@ __global__ void __launch_bounds__(C2P_THREADS, c2p_minb(MINK, kC2PFast)) kb_c2p(
   if (stats) c2p_flush_stats(stats, s_hist, s_cnt);
 }
 
-template <bool MINK>
+template <bool MINK, bool RHOU>
 static void c2p_batched_t(const Par &p, const BView *views, const WorkItem *items, int nitems, int grid,
                           const MlpPacked *mlp, double *brk, DevStats *stats, unsigned int *err, cudaStream_t s) {
+  const auto plain = kb_c2p<MINK, false, RHOU>, cold = kb_c2p<MINK, true, RHOU>;
+  const int plain_grid = persistent_grid(plain, C2P_THREADS, 0, nitems, grid);
   if (mlp) {
     static_assert(sizeof(BracketSmem) <= 48 * 1024, "no opt-in attribute needed (launches may be captured)");
     // warm pass (classifies and counts), bracket kernel, cold pass
     cudaMemsetAsync(brk + 4 * (long long)nitems * C2P_THREADS, 0, sizeof(unsigned long long), s);
-    kb_c2p<MINK, false><<<persistent_grid(kb_c2p<MINK, false>, C2P_THREADS, 0, nitems, grid), C2P_THREADS, 0, s>>>(
-        p, views, items, nitems, brk, stats, err, 1);
+    plain<<<plain_grid, C2P_THREADS, 0, s>>>(p, views, items, nitems, brk, stats, err, 1);
     kb_mlp_bracket<MINK><<<persistent_grid(kb_mlp_bracket<MINK>, C2P_THREADS, sizeof(BracketSmem), nitems, 0),
                            C2P_THREADS, sizeof(BracketSmem), s>>>(p, views, items, nitems, mlp, brk, err);
-    kb_c2p<MINK, true><<<persistent_grid(kb_c2p<MINK, true>, C2P_THREADS, 0, nitems, grid), C2P_THREADS, 0, s>>>(
-        p, views, items, nitems, brk, stats, err, 2);
+    cold<<<persistent_grid(cold, C2P_THREADS, 0, nitems, grid), C2P_THREADS, 0, s>>>(p, views, items, nitems, brk,
+                                                                                      stats, err, 2);
   } else {
-    kb_c2p<MINK, false><<<persistent_grid(kb_c2p<MINK, false>, C2P_THREADS, 0, nitems, grid), C2P_THREADS, 0, s>>>(
-        p, views, items, nitems, nullptr, stats, err, 0);
+    plain<<<plain_grid, C2P_THREADS, 0, s>>>(p, views, items, nitems, nullptr, stats, err, 0);
   }
 }
 
@@ -732,6 +741,7 @@ static void c2p_batched_t(const Par &p, const BView *views, const WorkItem *item
 // primitives it left, and prim2con with the zone's own metric (conserved
 // variables and cell speeds).  Item zone t of a block is the slab zone
 // i = n1t - ng + t % ng, j = (t / ng) % n2t, k = t / (ng n2t).
+template <bool RHOU>
 __global__ void __launch_bounds__(C2P_THREADS) kb_ox1_inflow(Par p, const BView *views, const WorkItem *items,
                                                               int nitems, unsigned int *err) {
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
@@ -754,7 +764,7 @@ __global__ void __launch_bounds__(C2P_THREADS) kb_ox1_inflow(Par p, const BView 
       setup_ok = c2p_setup<false>(p, g, U, x1, x2, x3, res, rcon, rcov, bu, Bprim, bdotr, flr);
     }
     C2POut out{0, 0, false, true, false, false};
-    const double mu = c2p_root_warp<false>(p, res, valid && setup_ok, guess, out);
+    const double mu = c2p_root_warp<false, RHOU>(p, res, valid && setup_ok, guess, out);
     if (!valid) continue;
     c2p_complete<BoxZones, false>(p, zones, id, g, res, mu, rcon, bu, Bprim, bdotr, U, setup_ok, out, err);
     double *P = bv.prim + id;
@@ -781,17 +791,16 @@ __global__ void __launch_bounds__(C2P_THREADS) kb_ox1_inflow(Par p, const BView 
 void launch_ox1_inflow(const Par &p, const BView *views, const WorkItem *items, int nitems, int grid,
                        unsigned int *err, cudaStream_t s) {
   if (nitems <= 0) return;
-  kb_ox1_inflow<<<persistent_grid(kb_ox1_inflow, C2P_THREADS, 0, nitems, grid), C2P_THREADS, 0, s>>>(
-      p, views, items, nitems, err);
+  const auto k = c2p_rhou(p) ? kb_ox1_inflow<kC2PFast> : kb_ox1_inflow<false>;
+  k<<<persistent_grid(k, C2P_THREADS, 0, nitems, grid), C2P_THREADS, 0, s>>>(p, views, items, nitems, err);
 }
 
 void launch_c2p_batched(const Par &p, bool mink, const BView *views, const WorkItem *items, int nitems, int grid,
                         const MlpPacked *mlp, double *brk, DevStats *stats, unsigned int *err, cudaStream_t s) {
   if (nitems <= 0) return;
-  if (mink)
-    c2p_batched_t<true>(p, views, items, nitems, grid, mlp, brk, stats, err, s);
-  else
-    c2p_batched_t<false>(p, views, items, nitems, grid, mlp, brk, stats, err, s);
+  const auto launch = c2p_rhou(p) ? (mink ? c2p_batched_t<true, kC2PFast> : c2p_batched_t<false, kC2PFast>)
+                                  : (mink ? c2p_batched_t<true, false> : c2p_batched_t<false, false>);
+  launch(p, views, items, nitems, grid, mlp, brk, stats, err, s);
 }
 
 }  // namespace phx

@@ -579,6 +579,9 @@ __device__ __forceinline__ FF ff_bits(double x) {
 //   eval:  FP32 and the derivative
 //   evalp: pairs of floats
 //   eval64: FP64; 38 arithmetic instructions and integer comparisons
+// RHOU: the energy floor follows the density (ExpX1RhoU); code of its own, whose
+// size costs the other floors' kernels 2 to 5%.
+template <bool RHOU>
 struct FastResidual {
   FF q, hb, rsq, rbsq, v0sq, gm1, bsq;  // q: q - bsq / 2, hb: -bsq_rpsq / 2
   float efl, emax;
@@ -594,13 +597,28 @@ struct FastResidual {
     rbsq = ff_bits(r.rbsq);
     v0sq = ff_bits(r.v0sq);
     gm1 = ff_bits(p.gm1);
-    double rho = r.rho_floor;  // ExpX1RhoU: the sie floor at the density floor, its largest value
+    double rho = r.rho_floor;  // RHOU: the sie floor at the density floor, its largest value
     floors_from(p, r.fl, rho, efl64);
     efl64 *= p.fsf;
     efl = d2f_bits(efl64);
     emax = d2f_bits(r.e_max);
   }
-  __device__ __forceinline__ float eval(float mu, float &df) const {
+  // RHOU: the specific energy floor s / max(rho, r), rho = max(D / W, its floor);
+  // moving: it follows D / W here
+  __device__ __forceinline__ float rhou_floor(const Par &p, const Residual &r, float iW, bool &moving) const {
+    const float lo = d2f_bits(max_num(r.rho_floor, r.fl.r)), rho = d2f_bits(r.D) * iW, sc = d2f_bits(p.fsf);
+    const float ef = sc * d2f_bits(r.fl.s) * rcp_f32(fmaxf(rho, lo)), em = sc * d2f_bits(p.sie_min_eos);
+    moving = rho > lo && ef > em;
+    return fmaxf(ef, em);
+  }
+  __device__ __forceinline__ FF rhou_floor(const Par &p, const Residual &r, FF iW) const {
+    const FF lo = ff_bits(max_num(r.rho_floor, r.fl.r)), sc = ff_bits(p.fsf);
+    FF rho = ff_mul(ff_bits(r.D), iW);
+    if (lo.h > rho.h || (lo.h == rho.h && lo.l > rho.l)) rho = lo;
+    const FF ef = ff_mul(ff_mul(sc, ff_bits(r.fl.s)), ff_rcp(rho)), em = ff_mul(sc, ff_bits(p.sie_min_eos));
+    return em.h > ef.h ? em : ef;
+  }
+  __device__ __forceinline__ float eval(const Par &p, const Residual &r, float mu, float &df) const {
     const float x = rcp_f32(fmaf(mu, bsq.h, 1.0f));
     const float dx = -bsq.h * x * x;
     const float mr = mu * rbsq.h, u = rsq.h + mr;
@@ -622,8 +640,12 @@ struct FastResidual {
     const float dW = 0.5f * W * W * W * dv2, diW = -0.5f * W * dv2;
     float e = fmaf(W, A, W - 1.0f), de = fmaf(dW, A + 1.0f, W * dA);
     if (e <= efl) {
-      e = efl;
-      de = 0.0f;
+      bool moving = false;
+      const float ef = RHOU ? rhou_floor(p, r, iW, moving) : efl;
+      if (!RHOU || e <= ef) {
+        e = ef;
+        de = moving ? 0.5f * ef * W * W * dv2 : 0.0f;
+      }
     } else if (e > emax) {
       e = emax;
       de = 0.0f;
@@ -639,7 +661,7 @@ struct FastResidual {
     df = fmaf(g * g, dnu + dmrb, 1.0f);
     return mu - g;
   }
-  __device__ __forceinline__ float evalp(FF mu) const {
+  __device__ __forceinline__ float evalp(const Par &p, const Residual &r, FF mu) const {
     const FF x = ff_rcp(ff_addf(ff_mul(mu, bsq), 1.0f));
     const FF mr = ff_mul(mu, rbsq);
     const FF rb = ff_mul(x, ff_add(mr, ff_mul(x, ff_add(rsq, mr))));
@@ -652,7 +674,8 @@ struct FastResidual {
     const FF W = ff_rsqrt(om), iW = ff_mul(om, W);
     FF e = ff_add(ff_mul(W, A), ff_addf(W, -1.0f));
     if (e.h <= efl) {
-      e = {efl, 0.0f};
+      const FF ef = RHOU ? rhou_floor(p, r, iW) : FF{efl, 0.0f};
+      if (!RHOU || e.h < ef.h || (e.h == ef.h && e.l <= ef.l)) e = ef;
     } else if (e.h > emax) {
       e = {emax, 0.0f};
     }
@@ -663,8 +686,7 @@ struct FastResidual {
     return __fadd_rn(__fsub_rn(mu.h, g.h), __fsub_rn(mu.l, g.l));
   }
   // false (the reference's expressions apply): a density negative or small
-  // enough for the reference's bound on h rho, an energy below 0, ExpX1RhoU's
-  // floor active
+  // enough for the reference's bound on h rho, an energy below 0
   // room: about the relative change of mu that switches the velocity bound or
   // one of the energy bounds
   __device__ __forceinline__ bool eval64(const Par &p, const Residual &r, double mu, double &f, float &room) const {
@@ -683,10 +705,12 @@ struct FastResidual {
     if (dexp(e) == 0x7ff) return false;  // NaN or infinity
     const float ef = d2f_bits(e), Wf = d2f_bits(W);  // mu de/dmu is of size W (W (1 + e) + mrb + |A|)
     const float de = Wf * fmaf(Wf, 1.0f + fabsf(ef), d2f_bits(mrb) + fabsf(d2f_bits(A)));
-    room = fminf(0.5f * dv, fminf(fabsf(ef - efl), fabsf(ef - emax)) * rcp_f32(de));
-    if (!gt_bits(e, efl64)) {
-      if (p.floor_type == PHX_FLOOR_EXPX1_RHO_U) return false;
-      e = efl64;
+    double bound = efl64;
+    if constexpr (RHOU)
+      bound = p.fsf * max_num(r.fl.s * rcp_p(max_num(max_num(r.D * iW, r.rho_floor), r.fl.r)), p.sie_min_eos);
+    room = fminf(0.5f * dv, fminf(fabsf(ef - d2f_bits(bound)), fabsf(ef - emax)) * rcp_f32(de));
+    if (!gt_bits(e, bound)) {
+      e = bound;
     } else if (gt_bits(e, r.e_max)) {
       e = r.e_max;
     }
@@ -702,10 +726,10 @@ struct FastResidual {
 // mu of one zone from its guess (> 0: a previous solution) or, LEARNED, the
 // predicted root lb[0] of a cold zone.  False: not accepted.  mu lies within
 // c2p_tol of the root where true, as the reference's final bracket has it.
-template <bool LEARNED>
+template <bool LEARNED, bool RHOU>
 __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res, double guess, const double *lb,
                                               double &mu, C2POut &out) {
-  const FastResidual rf(p, res);
+  const FastResidual<RHOU> rf(p, res);
   float lo = 0.0f, hi = 1.0f, s = 1.0f;
   float m = guess > 0.0 && guess < 1.0 ? d2f_bits(guess) : rsqrt_f32(1.0f + rf.rsq.h);
   out.learned = false;
@@ -713,7 +737,7 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
     if (!(guess > 0.0) && lb[1] >= 0.0 && lb[1] <= lb[0] && lb[0] <= lb[2] && lb[2] <= 1.0) {
       float d;
       const float l = d2f_bits(lb[1]), h = d2f_bits(lb[2]);
-      if (rf.eval(l, d) <= 0.0f && rf.eval(h, d) >= 0.0f) {
+      if (rf.eval(p, res, l, d) <= 0.0f && rf.eval(p, res, h, d) >= 0.0f) {
         m = d2f_bits(lb[0]);
         lo = l;
         hi = h;
@@ -723,7 +747,7 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
   }
   float last = 1.0f, span = 1.0f;  // span: how far from the root the slope's points may lie
   for (int it = 0; it < 24; it++) {
-    const float f = rf.eval(m, s);
+    const float f = rf.eval(p, res, m, s);
     if (f > 0.0f)
       hi = m;
     else
@@ -744,7 +768,7 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
   float is = rcp_f32(s), step = 0.0f, fp = 0.0f;
 #pragma unroll 1
   for (int it = 0; it < 5; it++) {
-    const float f = rf.evalp(mp);
+    const float f = rf.evalp(p, res, mp);
     if (it > 0 && fabsf(step) > 1e-7f * m) {
       is = step * rcp_f32(fp - f);
       span = fabsf(step);
@@ -808,13 +832,13 @@ static __device__ __noinline__ double c2p_slow_root(const Par &p, Residual res, 
 
 // The root of one zone per lane, warp-synchronous: the production build's
 // fast root where it is accepted, the reference's iteration elsewhere.
-template <bool LEARNED>
+template <bool LEARNED, bool RHOU>
 __device__ __forceinline__ double c2p_root_warp(const Par &p, Residual &res, bool valid, double guess, C2POut &out,
                                                 const double *lb = nullptr) {
 #ifndef PHX_EXACT
   bool need = valid;
   double mu = guess;
-  if (valid && c2p_fast_allowed(p)) need = !c2p_fast_root<LEARNED>(p, res, guess, lb, mu, out);
+  if (valid && c2p_fast_allowed(p)) need = !c2p_fast_root<LEARNED, RHOU>(p, res, guess, lb, mu, out);
   if (!__any_sync(0xffffffffu, need)) return mu;
   C2POut slow{0, 0, false, true, false, false};
   double ms;

@@ -150,3 +150,22 @@ def test_learned_start_outside_the_fast_rule(ctx_fast, oracle, tol, max_iter, n)
     assert stats["residual_evals"] >= 3 * n  # no zone by the fast root
     if max_iter == 100:
         assert np.abs(got[abi.PMU] - mu).max() <= tol + 1e-13
+
+
+@pytest.mark.parametrize("gm1,rho0,sie0", [(1 / 3, 1e-3, 1e-3), (2 / 3, 1e-5, 1e-1), (1 / 3, 1e-6, 1e-6)])
+def test_density_dependent_energy_floor(ctx_fast, oracle, gm1, rho0, sie0):
+    """ExpX1RhoU's specific energy floor falls with the zone's density; where it
+    holds at the root the fast root still finds it: within the tolerance, the
+    same zones rewritten, one to three FP64 evaluations per zone."""
+    n, tol = 20_000, 1e-10
+    p = abi.default_params(gm1=gm1, c2p_tol=tol, c2p_max_iter=100)
+    prim = zone_prims(n, 35, gm1, 20.0)
+    cons = oracle.PrimitiveToConservedZones(p, prim)
+    cons[abi.CENG] *= np.where(np.arange(n) % 3 == 0, 0.97, 1.0)
+    p.enable_floors, p.floor_type, p.rho0_floor, p.sie0_floor = 1, abi.FLOOR["ExpX1RhoU"], rho0, sie0
+    ref, rfail, rc = reference(oracle, p, cons, prim * 0.0)
+    got, fail, c, stats = solve(ctx_fast, p, cons, prim * 0.0)
+    assert np.array_equal(fail, rfail)
+    assert np.abs(got[abi.PMU] - ref[abi.PMU]).max() <= 2.0 * tol + 1e-13
+    assert np.array_equal(np.any(c != cons, axis=0), np.any(rc != cons, axis=0))
+    assert n <= stats["residual_evals"] < 3 * n
