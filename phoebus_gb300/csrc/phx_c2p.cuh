@@ -4,9 +4,9 @@
 // The regula-falsi loop is warp-synchronous: every lane stays in the loop
 // until the warp's vote (__any_sync) says no lane is still iterating, so all
 // 32 lanes re-enter each iteration together and reconverge after it.
-// In the production build the residual's divisions use the Newton-refined
-// hardware reciprocal (rcp_p / ratio_p); the exact build divides as the
-// reference does.
+// In the production build the residual's divisions use the reciprocal on the
+// FP32 and integer pipes (rcp_p / ratio_p), and the fast root below comes first;
+// the exact build divides and iterates as the reference does.
 #pragma once
 #include "phx_device.cuh"
 
@@ -44,7 +44,9 @@ struct Residual {
     used_gamma_max = false;
     return vsq_trial;
   }
+#ifdef PHX_EXACT
   __device__ __forceinline__ double iWhat_mu(double vhatsq) const { return sqrt(1.0 - vhatsq); }
+#endif
   __device__ __forceinline__ double rhohat_mu(double iWhat) {
     const double rho_trial = D * iWhat;
     if (!gt(rho_trial, rho_floor) && !is_nan(rho_trial)) {
@@ -54,6 +56,7 @@ struct Residual {
     used_density_floor = false;
     return rho_trial;
   }
+#ifdef PHX_EXACT
   __device__ __forceinline__ double ehat_mu(const Par &p, double mu, double qbar, double rbarsq,
                                             double vhatsq, double What) {
     double rho = rhohat_mu(ratio_p(1.0, What));
@@ -72,6 +75,7 @@ struct Residual {
     }
     return ehat_trial;
   }
+#else
   // the energy bounds of ehat_mu at density rho (production build)
   __device__ __forceinline__ double bound_ehat(const Par &p, double rho, double ehat_trial) {
     double e_floor;
@@ -94,6 +98,7 @@ struct Residual {
                                                double What, double iWhat) {
     return bound_ehat(p, rhohat_mu(iWhat), fma(What, qbar - mu * rbarsq, What - 1.0));
   }
+#endif
   __device__ __forceinline__ double operator()(const Par &p, double mu) {
     const double x = x_mu(mu);
     const double rbarsq = rbarsq_mu(mu, x);

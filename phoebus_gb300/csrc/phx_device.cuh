@@ -618,12 +618,14 @@ __device__ __forceinline__ double mc(double dm, double dp, double alpha) {
   return copysign(fmin(fabs(dc), alpha * fmin(fabs(dm), fabs(dp))), dc);
 #endif
 }
+#ifdef PHX_EXACT
 __device__ __forceinline__ void recon_plm(double qm, double q0, double qp, double &ql, double &qr) {
   double dq = qp - q0;
   dq = mc(q0 - qm, dq, 1.5);
   ql = q0 + 0.5 * dq;
   qr = q0 - 0.5 * dq;
 }
+#else
 // Production PLM: 5 FP64 instructions.  With dm, dp of one sign, the halved
 // slope is min(|dm + dp| / 4, 3/4 min(|dm|, |dp|)), and the first is the
 // smaller exactly where the larger of |dm|, |dp| is below twice the other:
@@ -642,6 +644,7 @@ __device__ __forceinline__ void recon_plm_fast(double qm, double q0, double qp, 
   ql = fma(c, s, q0);
   qr = fma(-c, s, q0);
 }
+#endif
 __device__ __forceinline__ void recon_weno5z(double q0, double q1, double q2, double q3, double q4,
                                              double &ql, double &qr) {
   constexpr double a00 = 1.0 / 3.0, a01 = -7.0 / 6.0, a02 = 11.0 / 6.0;
@@ -744,6 +747,7 @@ __device__ __forceinline__ void recon_weno5z_fast(double q0, double q1, double q
   qr = w.mirror ? qa : qb;
 }
 
+#ifdef PHX_EXACT
 __device__ __forceinline__ double minmod(double a, double b) {
   return a * b > 0.0 ? (fabs(a) < fabs(b) ? a : b) : 0.0;
 }
@@ -759,11 +763,7 @@ __device__ __forceinline__ double minmod(double a, double b) {
 __device__ __forceinline__ double mp5_face(double fm2, double fm1, double f0, double fp1, double fp2) {
   constexpr double alpha = 4.0, eps = 1.e-12;
   double f = 2.0 * fm2 - 13.0 * fm1 + 47.0 * f0 + 27.0 * fp1 - 3.0 * fp2;
-#ifdef PHX_EXACT
   f /= 60.0;
-#else
-  f *= 1.0 / 60.0;  // a product instead of the IEEE division (an ulp apart)
-#endif
   const double f_mp = f0 + minmod(fp1 - f0, alpha * (f0 - fm1));
   if ((f - f0) * (f - f_mp) <= eps) return f;
   const double curv_m = fm2 + f0 - 2.0 * fm1;  // second differences at j-1, j, j+1
@@ -779,7 +779,7 @@ __device__ __forceinline__ double mp5_face(double fm2, double fm1, double f0, do
   const double f_max = fmin(fmax(fmax(f0, fp1), f_md), fmax(fmax(f0, f_ul), f_lc));
   return f + minmod(f_min - f, f_max - f);  // the median of f, f_min, f_max
 }
-
+#else
 // Both face values of a cell by the same scheme, in differences from f_j
 // (production build): 18 FP64 instructions, 29 where a face is limited
 // (38 and about 20 FP64 comparisons per face in mp5_face).  The two faces
@@ -821,6 +821,7 @@ __device__ __forceinline__ void recon_mp5_fast(double q0, double q1, double q2, 
   ql = q2 + gl;
   qr = q2 + gr;
 }
+#endif
 
 // 5-point (or 3-point) reconstruction of one variable.  ql = value at the
 // upper face of the cell, qr = value at its lower face.
@@ -861,7 +862,9 @@ struct Face {
   FloorPt fl;    // floor_point at the face, shared by its two states
 };
 
-// prim_to_flux (riemann.hpp:88-209) for face direction DIR (0-based).
+#ifdef PHX_EXACT
+// prim_to_flux (riemann.hpp:88-209) for face direction DIR (0-based), in the
+// reference's operations (exact build; flux_state in the production build).
 template <bool MINK, int DIR>
 __device__ __forceinline__ void prim_to_flux(const Par &par, const Face &f, const double q[PHX_NRECON],
                                              double &vm, double &vp, double U[PHX_NCONS],
@@ -872,43 +875,16 @@ __device__ __forceinline__ void prim_to_flux(const Par &par, const Face &f, cons
   floors_from(par, f.fl, rho_floor, sie_floor);
   const double rho = rmax(q[PHX_PRHO], rho_floor);
   double vpcon[3] = {q[PHX_PVEL], q[PHX_PVEL + 1], q[PHX_PVEL + 2]};
-#ifdef PHX_EXACT
   double W = lorentz<MINK>(g, vpcon);
-#else
-  const double Wsq0 = 1. + dot_sp<MINK>(g, vpcon, vpcon);
-  const double iW0 = rsqrt_p(Wsq0);
-  double W = Wsq0 * iW0;
-#endif
-#ifndef PHX_EXACT
-  bool capped = false;  // a velocity cap changed v: W is formed again below
-#endif
   if (W > gam_max) {
     const double rescale = sqrt((gam_max * gam_max - 1.) / (W * W - 1.));
 #pragma unroll
     for (int ii = 0; ii < 3; ii++) vpcon[ii] *= rescale;
-#ifndef PHX_EXACT
-    capped = true;
-#endif
   }
   const double qe = q[PHX_PENG];
-#ifdef PHX_EXACT
   double vcon[3] = {vpcon[0] / W, vpcon[1] / W, vpcon[2] / W};
   const double sie_q = q[PHX_PENG] / rho;
   const bool above_floor = sie_q > sie_floor, above_max = sie_q > sie_max;
-#else
-  double vcon[3] = {vpcon[0] * iW0, vpcon[1] * iW0, vpcon[2] * iW0};
-  // u / rho > s as u > rho s for rho > 0 (no reciprocal; the products are the
-  // bounded energies anyway); the quotient only where rho <= 0
-  bool above_floor, above_max;
-  if (rho > 0.0) {
-    above_floor = qe > rho * sie_floor;
-    above_max = qe > rho * sie_max;
-  } else {
-    const double sie_q = qe * rcp_p(rho);
-    above_floor = sie_q > sie_floor;
-    above_max = sie_q > sie_max;
-  }
-#endif
   double Bcon[3] = {0.0, 0.0, 0.0};
   const double u = (above_floor ? (above_max ? rho * sie_max : qe) : rho * sie_floor);
   const double P = rmax(q[PHX_PPRS], 0.0);
@@ -927,7 +903,6 @@ __device__ __forceinline__ void prim_to_flux(const Par &par, const Face &f, cons
     vsq = 0.0;
     Bdotv = 0.0;
     BdotB = 0.0;
-#ifdef PHX_EXACT
 #pragma unroll
     for (int m = 0; m < 3; m++)
 #pragma unroll
@@ -936,25 +911,8 @@ __device__ __forceinline__ void prim_to_flux(const Par &par, const Face &f, cons
         Bdotv += g.gcov[m + 1][n + 1] * Bcon[m] * vcon[n];
         BdotB += g.gcov[m + 1][n + 1] * Bcon[m] * Bcon[n];
       }
-#endif
   }
-#ifndef PHX_EXACT
-  // production build: the lowered v and B serve the three contractions here
-  // and the covariant momentum / field terms below
-  double vlo[3], Blo[3];
-  if constexpr (!MINK) {
-    lower_sp(g, vcon, vlo);
-    lower_sp(g, Bcon, Blo);
-    vsq = dot3(vcon, vlo);
-    Bdotv = dot3(Bcon, vlo);
-    BdotB = dot3(Bcon, Blo);
-  }
-#endif
-#ifdef PHX_EXACT
   const double vsq_max = 1.0 - 1.0 / (gam_max * gam_max);
-#else
-  const double vsq_max = par.vsq_max;  // 1 - 1 / gam_max^2, formed on the host
-#endif
   if (vsq > vsq_max) {
     double scale = vsq_max / vsq;
     vsq *= scale;
@@ -962,33 +920,11 @@ __device__ __forceinline__ void prim_to_flux(const Par &par, const Face &f, cons
     Bdotv *= scale;
 #pragma unroll
     for (int m = 0; m < 3; m++) vcon[m] *= scale;
-#ifndef PHX_EXACT
-    if constexpr (!MINK)
-#pragma unroll
-      for (int m = 0; m < 3; m++) vlo[m] *= scale;
-    capped = true;
-#endif
   }
-#ifdef PHX_EXACT
   W = 1.0 / sqrt(1 - vsq);
-#else
-  // production build: W = 1/s with s = sqrt(1 - v^2); divisions by W and W^2
-  // become products with s and s^2.  Without a cap v^2 = 1 - 1/W0^2, so W
-  // stays W0 and s is the 1/W0 formed above (no second rsqrt)
-  double sW = iW0;
-  if (capped) {
-    W = rsqrt_p(1 - vsq);
-    sW = (1 - vsq) * W;
-  }
-#endif
   const double vel = vcon[DIR];
   const double alpha = MINK ? 1.0 : g.alpha;
-#ifdef PHX_EXACT
 #define PHX_BOA(m) (g.beta[m] / alpha)
-#else
-  const double ialpha = MINK ? 1.0 : rcp_p(alpha);
-#define PHX_BOA(m) (g.beta[m] * ialpha)
-#endif
   double vtil;
   if constexpr (MINK)
     vtil = vel;
@@ -997,32 +933,19 @@ __device__ __forceinline__ void prim_to_flux(const Par &par, const Face &f, cons
   U[PHX_CRHO] = rho * W;
   F[PHX_CRHO] = U[PHX_CRHO] * vtil;
   const double b0 = W * Bdotv;
-#ifdef PHX_EXACT
   const double bsq = (BdotB + b0 * b0) / (W * W);
   const double rhohWsq = (rho + u + P) * W * W;
   const double bsqWsq = bsq * W * W;
-#else
-  // production build: bsq W^2 = B.B + b0^2 (sW = 1/W), W^2 formed once
-  const double Wsq = W * W;
-  const double bsqWsq = fma(b0, b0, BdotB);
-  const double bsq = bsqWsq * (sW * sW);
-  const double rhohWsq = (rho + u + P) * Wsq;
-#endif
   const double ptot = P + 0.5 * bsq;
 #pragma unroll
   for (int m = 0; m < 3; m++) {
     double bcovm, vcovm;
-#ifdef PHX_EXACT
 #define PHX_DIV_W(x) ((x) / W)
-#else
-#define PHX_DIV_W(x) ((x) * sW)
-#endif
     if constexpr (MINK) {
       // gcov[m+1][0] = 0: first term is +-0; then only n = m+1 survives
       bcovm = PHX_DIV_W(Bcon[m]) + b0 * vcon[m];
       vcovm = vcon[m];
     } else {
-#ifdef PHX_EXACT
       bcovm = g.gcov[m + 1][0] * b0 / alpha;
       vcovm = 0.0;
 #pragma unroll
@@ -1030,68 +953,30 @@ __device__ __forceinline__ void prim_to_flux(const Par &par, const Face &f, cons
         bcovm += g.gcov[m + 1][n] * (PHX_DIV_W(Bcon[n - 1]) + b0 * (vcon[n - 1] - PHX_BOA(n - 1)));
         vcovm += g.gcov[m + 1][n] * vcon[n - 1];
       }
-#else
-      // g_{m0} = gamma_mn beta^n: the shift terms cancel, b_m = B_m / W + b0 v_m
-      bcovm = Blo[m] * sW + b0 * vlo[m];
-      vcovm = vlo[m];
-#endif
     }
     U[PHX_CMOM + m] = (rhohWsq + bsqWsq) * vcovm - b0 * bcovm;
     F[PHX_CMOM + m] = U[PHX_CMOM + m] * vtil + ptot * (double)(DIR == m) - PHX_DIV_W(bcovm * Bcon[DIR]);
 #undef PHX_DIV_W
   }
-#ifdef PHX_EXACT
   U[PHX_CENG] = rhohWsq + bsqWsq - ptot - b0 * b0 - U[PHX_CRHO];
-#else
-  U[PHX_CENG] = rhohWsq + BdotB - ptot - U[PHX_CRHO];  // bsq W^2 - b0^2 = B.B
-#endif
   F[PHX_CENG] = U[PHX_CENG] * vtil + ptot * vel - Bdotv * Bcon[DIR];
 #pragma unroll
   for (int m = 0; m < 3; m++) {
     U[PHX_CB + m] = Bcon[m];
     if constexpr (MINK) {
-#ifdef PHX_EXACT
       F[PHX_CB + m] = U[PHX_CB + m] * vtil - Bcon[DIR] * vcon[m];
-#else
-      // production build: B^d v^d - B^d v^d is 0 as the reference computes it
-      // (equal products); contracted into an FMA it would be the product's
-      // rounding error instead
-      F[PHX_CB + m] = m == DIR ? 0.0 : U[PHX_CB + m] * vtil - Bcon[DIR] * vcon[m];
-#endif
     } else {
       F[PHX_CB + m] = U[PHX_CB + m] * vtil - Bcon[DIR] * (vcon[m] - PHX_BOA(m));
     }
   }
 #undef PHX_BOA
-#ifdef PHX_EXACT
   const double vasq = bsqWsq / make_positive(rhohWsq + bsqWsq);
   const double cssq = make_bounded(gamma1 * P * W * W / make_positive(rhohWsq), 0.0, 1.0);
-#else
-  // one reciprocal of the product of the two denominators when it is normal
-  const double dA = make_positive(rhohWsq + bsqWsq), dB = make_positive(rhohWsq);
-  const double dAB = dA * dB;
-  const int eAB = dexp(dAB);
-  double vasq, cs_raw;
-  if (eAB >= 16 && eAB <= 2030) {
-    const double rAB = rcp_nr(dAB);
-    vasq = bsqWsq * (dB * rAB);
-    cs_raw = gamma1 * P * Wsq * (dA * rAB);
-  } else {
-    vasq = bsqWsq * rcp_p(dA);
-    cs_raw = gamma1 * P * Wsq * rcp_p(dB);
-  }
-  const double cssq = make_bounded(cs_raw, 0.0, 1.0);
-#endif
   const double cmsq = make_bounded(cssq + vasq * (1.0 - cssq), 0.0, 1.0);
   const double vcoff = div_p(alpha, 1.0 - vsq * cmsq);
   const double v0 = vel * (1.0 - cmsq);
   const double gdd = MINK ? 1.0 : f.gdd;
-#ifdef PHX_EXACT
   const double vpm = sqrt(make_positive(cmsq * (1.0 - vsq) * (gdd * (1.0 - vsq * cmsq) - vel * v0)));
-#else
-  const double vpm_sq = make_positive(cmsq * (1.0 - vsq) * (gdd * (1.0 - vsq * cmsq) - vel * v0));
-  const double vpm = vpm_sq * rsqrt_p(vpm_sq);  // vpm_sq >= 10 DBL_EPSILON > 0
-#endif
   vp = vcoff * (v0 + vpm);
   vm = vcoff * (v0 - vpm);
   if constexpr (!MINK) {
@@ -1099,8 +984,7 @@ __device__ __forceinline__ void prim_to_flux(const Par &par, const Face &f, cons
     vm -= g.beta[DIR];
   }
 }
-
-#ifndef PHX_EXACT
+#else
 // Production build of one face state: prim_to_flux with the flux left as
 // F_m = U_m vtil + G_m, so that the Riemann combination applies vtil once per
 // state instead of once per variable, comparisons on the integer pipe, and
