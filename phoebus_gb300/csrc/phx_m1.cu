@@ -481,10 +481,13 @@ struct Closure {
     if (e >= 16 && e <= 2030) {
       im = rsqrt_nr(m2);
       xi = smax(smin(1.0, ratio_p(m2 * im, J)), 0.0);
-    } else if (__double_as_longlong(m2) > 0) {
+    } else if (__double_as_longlong(m2) > 0 && e < 0x7ff) {
       const double h = sqrt(m2);
       im = 1.0 / h;
       xi = smax(smin(1.0, ratio_p(h, J)), 0.0);
+    } else if (__double_as_longlong(m2) == 0x7ff0000000000000ll) {  // the square overflowed
+      im = 0.0;
+      xi = 1.0;
     } else {
       im = xi = __double_as_longlong(m2) == 0 ? 0.0 : __longlong_as_double(0x7ff8000000000000ll);
     }
