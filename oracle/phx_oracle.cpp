@@ -1463,7 +1463,7 @@ long long apply_floors(const phx_params &par, const phx_block *blk, phx_range ib
         auto P = [&](int v) -> Real & { return B.P(v, k, j, i); };
         auto U = [&](int v) -> Real & { return B.U(v, k, j, i); };
         const Real x1 = B.Xc(1, i), x2 = B.Xc(2, j), x3 = B.Xc(3, k);
-        Real rho_floor, sie_floor;
+        Real rho_floor = 0.0, sie_floor;  // uninitialised in the reference (read by ExpX1RhoU)
         bounds.GetFloors(x1, x2, x3, rho_floor, sie_floor);
         Real gamma_max, e_max;
         bounds.GetCeilings(x1, x2, x3, gamma_max, e_max);

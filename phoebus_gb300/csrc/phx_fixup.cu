@@ -136,7 +136,9 @@ __device__ __forceinline__ void floors_at(const Par &p, const BView &b, const Ra
     x1 = b.Xc(0, i);
     x2 = b.Xc(1, j);
     x3 = b.Xc(2, k);
-    double rho_floor, sie_floor;
+    // ExpX1RhoU reads a density here, which the reference leaves uninitialised: 0, as
+    // its other calls pass, so the energy floor is a floor-density zone's
+    double rho_floor = 0.0, sie_floor;
     flr = floor_cell(b, i);
     floors_from(p, flr ? floor_load(flr) : floor_point(p, x1, x2, x3), rho_floor, sie_floor);
     const double e_max = p.smax0;
