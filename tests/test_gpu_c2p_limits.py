@@ -108,7 +108,7 @@ def test_bound_switching_beside_the_root(ctx_fast, oracle, tol, bound):
     assert not over.any(), (int(over.sum()), np.abs(got[abi.PMU] - ref[abi.PMU]).max() / tol)
 
 
-@pytest.mark.parametrize("floor", [0.0, 1e-18])
+@pytest.mark.parametrize("floor", [0.0, 1e-18, 1e-8])
 @pytest.mark.parametrize("sign_tau", [1.0, -1.0])
 def test_negative_density(ctx_fast, oracle, floor, sign_tau):
     """D < 0 (an update that overshot): the density is the floor, and where
