@@ -792,7 +792,7 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
   if (!(is > 0.0f && is < 1e3f)) return false;
   double x = f2d_bits(mp.h) + f2d_bits(mp.l);
   const float tol = d2f_bits(p.c2p_tol);
-  const float tight = fmaxf(0.125f * tol, fminf(tol, 1e-12f * m));  // the residual's rounding is of that size
+  const float tight = fmaxf(0.0625f * tol, fminf(tol, 1e-12f * m));  // the residual's rounding is of that size
   float f = 0.0f;
   out.iterations = out.evals = 0;
 #pragma unroll 1
@@ -820,8 +820,8 @@ __device__ __forceinline__ bool c2p_fast_root(const Par &p, const Residual &res,
     // Two secants that agree say nothing about the slope beyond the root, where
     // the residual has its kink (nua = nub, slopes up to 1.9 apart: an error
     // below the step).  Where a bound switches within reach of the points the
-    // slope comes from, slopes up to 6 apart were seen: the step has to be an
-    // eighth of the tolerance.
+    // slope comes from, slopes up to 12 apart were seen: the step has to be a
+    // sixteenth of the tolerance.
     if (fabsf(step) <= (room * m > 2.0f * span ? tol : tight)) {
       mu = x < 1.0 ? x : 1.0;
       return x > 0.0;
