@@ -849,7 +849,11 @@ def main():
     fp64 = None
     if prof.exists():
         d = json.loads(prof.read_text())
-        flops = d["fp64_flops_per_call_per_zone"] * zones
+        # the counts go with the faces computed (n + 1 along each direction, n + 2
+        # across it), of which a larger block has fewer per zone than the counted one
+        faces = lambda m: (m + 1) * (m + 2) ** 2 / m ** 3  # noqa: E731
+        counted = zones * faces(n) / faces(d["counted_n"])
+        flops = d["fp64_flops_per_call_per_zone"] * counted
         fp64 = {"achieved_tflops": flops / (flux_ms * 1e-3) / 1e12, "peak_tflops": fp64_peak / 1e12,
                 "frac": flops / (flux_ms * 1e-3) / fp64_peak, "flops_source": d["source"],
                 "peak_source": "measured in-process (phx_probe_fp64_peak)"}
@@ -857,7 +861,7 @@ def main():
             # the probe issues DFMAs only (2 flops each): its instruction rate is peak / 2.  A kernel
             # with DADD/DMUL in its mix reaches frac < 1 at the full issue rate; issue_frac is the
             # FP64 instruction rate against the probe's.
-            inst = d["fp64_instructions_per_call_per_zone"] * zones
+            inst = d["fp64_instructions_per_call_per_zone"] * counted
             fp64["issue_frac"] = inst / (flux_ms * 1e-3) / (fp64_peak / 2.0)
             fp64["instructions_source"] = d["instructions_source"]
     traffic = None

@@ -187,15 +187,22 @@ typedef struct {
 } phx_block;
 
 /* con2prim statistics, accumulated on the device by every con2prim call
- * (the reference's CON2PRIM_STATISTICS histogram, con2prim_statistics.hpp). */
+ * (the reference's CON2PRIM_STATISTICS histogram, con2prim_statistics.hpp).
+ * The exact build counts the reference's root-find iterations.  In the
+ * production build a zone that its fast root solves counts the FP64 residual
+ * evaluations that finished it (mostly 1) as iterations and as evaluations; a
+ * zone left to the reference's iteration counts that iteration's, and so do all
+ * zones with c2p_tol outside [1e-15, 1e-3] or c2p_max_iter below 5.  Sums and
+ * histogram there mix the two units. */
 #define PHX_C2P_HIST 128
 typedef struct {
   unsigned long long zones;
-  unsigned long long iterations;     /* sum of root-find iterations      */
+  unsigned long long iterations;     /* sum of root-find iterations (above) */
   unsigned long long residual_evals; /* sum of residual evaluations      */
   unsigned long long failures;       /* zones flagged fail = 0.0         */
   unsigned long long unbracketed;    /* zones whose root was not bracketed */
-  unsigned long long learned_accepted; /* learned brackets that bracketed */
+  unsigned long long learned_accepted; /* learned brackets that bracketed (fast
+                                        * root: by their ends in FP32) */
   unsigned long long hist[PHX_C2P_HIST]; /* iteration-count histogram     */
 } phx_c2p_stats;
 
@@ -234,8 +241,9 @@ phx_status phx_con_to_prim(phx_ctx *ctx, const phx_params *p, const phx_block *b
                            phx_range ib, phx_range jb, phx_range kb, void *stream);
 
 /* Same as phx_con_to_prim, but the starting bracket comes from the learned
- * guess network loaded into ctx (phx_mlp_set_weights).  The FP64 root find
- * and its fallback to the reference bracket are unchanged. */
+ * guess network loaded into ctx (phx_mlp_set_weights).  The root is the one
+ * phx_con_to_prim finds, within the same tolerance; a bracket that is not
+ * accepted leaves the start as it is there. */
 phx_status phx_con_to_prim_learned(phx_ctx *ctx, const phx_params *p, const phx_block *b,
                                    phx_range ib, phx_range jb, phx_range kb,
                                    void *stream);
@@ -471,10 +479,15 @@ phx_status phx_batch_info(phx_ctx *ctx, int *x1_cells, int *sweep_seg, int *grap
  * layer.  Outputs: o0 = predicted ln(mu), o1 = ln(sigma) of its error, mu the
  * con2prim unknown 1 / (h W).  The learned start is the bracket
  * [e^{o0 - 3 s}, e^{o0 + 3 s}] (s = e^{o1}, clipped to [0, 1]) around
- * m = e^{o0}; the root find evaluates f(m), then the outer end of the half
+ * m = e^{o0}.  Exact build, and c2p_tol or c2p_max_iter outside the fast
+ * root's range: the root find evaluates f(m), then the outer end of the half
  * that should hold the root, and starts the reference's Illinois iterations
  * from that half if it changes sign -- otherwise from the reference's own
- * [0, 1] + guess start.  Inference multiplies BF16 weights and activations on
+ * [0, 1] + guess start.  Production build otherwise: the residual at both ends
+ * is tested in FP32, m and the bracket start the FP32 search where they have
+ * opposite signs, and FP64 evaluations finish it as from any other start; no
+ * Illinois iteration follows, and one FP64 evaluation is usual with or without
+ * the network.  Inference multiplies BF16 weights and activations on
  * the tensor cores with FP32 accumulation. */
 
 /* Load FP32 master parameters (host memory, PHX_MLP_NPARAM floats); resets
