@@ -483,12 +483,12 @@ __host__ __device__ __forceinline__ bool c2p_fast_allowed(const Par &p) {
 // evaluation corrects that value; the correction times the slope's own
 // error is what is left, and the zone is accepted when it is below the
 // caller's tolerance (otherwise secant steps with further FP64 evaluations
-// follow).  A zone that does not pass these tests (floors or caps switching
-// at the root, values outside the FP32 range, NaN) takes the reference's
+// follow).  A zone that does not pass these tests (values outside the FP32
+// range, a density below 1e-14, NaN, no convergence) takes the reference's
 // bracketed iteration instead.
 // Measured against the bracketed iteration in FP64 (GB300, with the reciprocals
 // on the integer pipe and c2p_finish's algebra): 1.2e7 cold Kerr-Schild zones
-// at tolerance 1e-13 30.0 -> 5.6 ms (12.8 -> 1.05 FP64 residual evaluations per
+// at tolerance 1e-13 30.0 -> 5.5 ms (12.8 -> 1.01 FP64 residual evaluations per
 // zone), a 136^3 Minkowski block from stale mu 3.90 -> 0.87 ms (7.0 -> 1.0
 // evaluations; 147 FP64 instructions per zone, the FP64 pipe busy 94% of the
 // time), 1000 cold zones 96 -> 40 us; the root's error against the sampled
